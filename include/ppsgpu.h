@@ -107,7 +107,9 @@ typedef struct {
   uint32_t batches;     /* device batches used */
   uint32_t variant;     /* walk kernel variant used */
   double   sieve_ms, walk_ms, filter_ms, total_ms;  /* device time per phase */
-  uint32_t split;       /* threads per prime of the walk (the tuner's choice, 1..8) */
+  uint32_t split;       /* parts of each prime's n range walked side by side: threads per
+                           prime (the tuner's choice, 1..8), or the tensor walk's rows
+                           (128 per unit of work) */
   uint32_t reserved;
 } pps_job_stats;
 
@@ -158,7 +160,7 @@ int pps_engine_sm_count(const pps_engine *e);
 int pps_engine_set_batch_span(pps_engine *e, uint64_t span);
 
 /* Force a walk kernel variant (0..PPS_NUM_VARIANTS-1), or -1 for the tuned one. */
-#define PPS_NUM_VARIANTS 31
+#define PPS_NUM_VARIANTS 33
 int pps_engine_set_variant(pps_engine *e, int variant);
 
 /* A walk variant's short description ("queue2-min-u8": queued walk, two primes

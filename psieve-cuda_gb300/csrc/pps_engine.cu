@@ -23,6 +23,7 @@
 
 #include "pps_engine_impl.h"
 #include "pps_internal.h"
+#include "pps_tensor.cuh"
 #include "ppsgpu.h"
 
 using namespace pps;
@@ -173,6 +174,7 @@ static void free_engine(pps_engine* e) {
   e->presieve.release();
   e->sieve_res.release();
   e->probe_sink.release();
+  e->masks.release();
   batch_state_free(e);
   if (e->h_pinned) cudaFreeHost(e->h_pinned);
   for (auto& v : e->ev)
@@ -248,7 +250,7 @@ extern "C" uint64_t pps_engine_device_bytes(const pps_engine* e) {
   return e->base_q.bytes() + e->seed_q.bytes() + e->bitmap.bytes() + e->seg_count.bytes() +
          e->seg_off.bytes() + e->P.bytes() + e->Pinv.bytes() + e->totals.bytes() + e->hits.bytes() +
          e->factors.bytes() + e->counters.bytes() + e->small_q.bytes() + e->probe_sink.bytes() +
-         e->presieve.bytes() + e->sieve_res.bytes();
+         e->presieve.bytes() + e->sieve_res.bytes() + e->masks.bytes();
 }
 
 extern "C" int pps_engine_sm_count(const pps_engine* e) { return e ? e->num_sms : 0; }
@@ -489,6 +491,15 @@ static int variant_ok(const pps_job_params* jp, int v) {
   // the twin variants walk both sides of a twin job; every other variant one side
   const bool twin = jp->sign == PPS_SIGN_TWIN;
   if (twin != t.twin) return 0;
+  if (t.tensor) {
+    TensorPlan plan;
+    if (!tensor_plan(jp, &plan)) return 0;
+    if (!twin) return 1;
+    // twin jobs run where a recurrence kernel could walk them too
+    for (int w = 0; w < VARIANT_TENSOR; ++w)
+      if (variant_ok(jp, w)) return 1;
+    return 0;
+  }
   if (t.lowbit && jp->kmax >= (1ull << 32)) return 0;  // low-bit test needs kmax < 2^32
   if (t.s32 && jp->step != 32) return 0;
   if (t.shifted || t.smallp || t.min_window) {
@@ -601,7 +612,7 @@ static uint64_t variant_set(const pps_job_params* jp) {
   const double nsteps_full = jp->nmax > jp->nmin ? (double)((jp->nmax - jp->nmin + jp->step - 1) / jp->step) : 0.0;
   uint64_t exact = 0, cls = 0;
   for (int v = 0; v < PPS_NUM_VARIANTS; ++v)
-    if (variant_ok(jp, v)) {
+    if (!walk_variant_traits(v).tensor && variant_ok(jp, v)) {  // (the tensor walk has its own rule, tensor_choice)
       const VariantTraits& t = walk_variant_traits(v);
       exact |= 1ull << v;
       const double r = pretest_pass_rate(jp, v);
@@ -683,10 +694,51 @@ static int autotune(pps_engine* e, const pps_job_params* jp, const uint64_t* dP,
   return best;
 }
 
-static int ceil_lg(uint64_t x) {
-  int r = 0;
-  while ((1ull << r) < x && r < 63) r++;
-  return r;
+// Whether the job runs on the tensor walk, and how: where its cost is estimated
+// to be below the recurrence's, both in SM clocks per prime.  tensor_plan's
+// estimate holds within 8%.  The recurrence's is its steps times what one took
+// with 1.5 to 2.4 million primes: 32-bit steps 0.106-0.110 (p up to 2^50;
+// 0.089 at 2^62), shorter ones 0.135, a twin step 0.19-0.24 (on the batched
+// form).  On either side of the line: p = 4.2e13, N = 200,000: 693 clocks
+// against the tensor walk's 793, N = 300,000: 1,032 against 915; p = 2^62, N =
+// 300,000: 852 against 903, N = 600,000: 1,685 against 1,337; p = 10^12, N =
+// 150,000: 764 against 797, N = 200,000: 1,012 against 826.
+static bool tensor_choice(const pps_engine* e, const pps_job_params* jp, TensorPlan* plan) {
+  const bool twin = jp->sign == PPS_SIGN_TWIN;
+  const int v = twin ? VARIANT_TENSOR_TWIN : VARIANT_TENSOR;
+  if (e->forced_variant >= 0 && e->forced_variant != v && variant_ok(jp, e->forced_variant)) return false;
+  if (e->forced_split > 0 && e->forced_variant != v) return false;  // parts of the queued walks
+  if (e->forced_variant == v) return variant_ok(jp, v) && tensor_plan(jp, plan);
+  const double nsteps = (double)((jp->nmax - jp->nmin + jp->step - 1) / jp->step);
+  if (nsteps * 0.19 < TW_LEAST_COST) return false;  // (most short jobs, without the search for a plan)
+  return variant_ok(jp, v) && tensor_plan(jp, plan) &&
+         plan->cost < nsteps * (twin ? 0.19 : jp->step < 32 ? 0.135 : plan->digits == 4u ? 0.106 : 0.089);
+}
+
+static int run_tensor_walk(pps_engine* e, const pps_job_params* jp, const TensorPlan& plan, const uint64_t* dP,
+                           const uint64_t* dPinv, uint64_t np) {
+  if (int rc = e->masks.ensure(tensor_masks(plan, np))) return rc;
+  TensorArgs a;
+  a.P = dP;
+  a.Pinv = dPinv;
+  a.np = np;
+  a.pmin = jp->pmin;
+  a.pmax = jp->pmax;
+  a.kmin = jp->kmin;
+  a.kmax = jp->kmax;
+  a.nmin = jp->nmin;
+  a.nmax = jp->nmax;
+  a.side = jp->sign == PPS_SIGN_TWIN ? 2u : jp->sign == 1 ? 1u : 0u;
+  a.idx_base = 0;
+  a.plan = plan;
+  a.batch = 0;
+  a.work = e->counters.p + CNT_TENSOR;
+  a.hits = e->hits.p;
+  a.hit_count = e->counters.p;
+  a.hit_cap = hit_cap_now(e);
+  a.masks = e->masks.p;
+  CU(launch_tensor_walk(a, e->num_sms, e->st, &e->launches));
+  return PPS_OK;
 }
 
 // Threads per prime for the queued walk v on np primes (1 where the walk is not
@@ -754,12 +806,22 @@ extern "C" int pps_engine_set_input(pps_engine* e, const pps_input* in) {
   return PPS_OK;
 }
 
+// The tensor walk's status words in the pinned copy of the counters: an error
+// where a bounded wait ran out; *outside is set where the caller's list held a
+// prime outside the job's range (that walk leaves it out).
+static int tensor_status(const pps_engine* e, bool* outside) {
+  const uint32_t* c = (const uint32_t*)e->h_pinned + CNT_TENSOR;
+  if (c[2]) return set_err(PPS_ERR_TIMEOUT, "tensor walk: a bounded device wait expired");
+  if (c[1] && outside) *outside = true;
+  return PPS_OK;
+}
+
 // Filter the raw hits accumulated in e->hits and copy the factors out.
 // The filter runs on the device-side count of raw hits (clamped to the
 // buffer), so the two counts come back in one copy after it: a raw count
 // beyond the buffer then means an overflow (the call walks again).
 static int finish_job(pps_engine* e, const pps_job_params* jp, pps_factor* out, size_t cap, size_t* nout,
-                      pps_job_stats* st, uint32_t* raw_hits_out, bool* overflow) {
+                      pps_job_stats* st, uint32_t* raw_hits_out, bool* overflow, bool* outside = nullptr) {
   if (int rc = ensure_input_keys(e, jp)) return rc;
   FilterArgs f;
   f.hits = e->hits.p;
@@ -788,8 +850,10 @@ static int finish_job(pps_engine* e, const pps_job_params* jp, pps_factor* out, 
   CU(launch_filter(f, (uint32_t)e->num_sms * 8u, e->st));
   e->launches++;
   CU(cudaEventRecord(e->ev[5], e->st));
-  CU(cudaMemcpyAsync(e->h_pinned, e->counters.p, 2 * sizeof(uint32_t), cudaMemcpyDeviceToHost, e->st));
+  CU(cudaMemcpyAsync(e->h_pinned, e->counters.p, CNT_WORDS * sizeof(uint32_t), cudaMemcpyDeviceToHost, e->st));
   CU(cudaStreamSynchronize(e->st));
+  if (int rc = tensor_status(e, outside)) return rc;
+  if (outside && *outside) return PPS_OK;  // the caller walks its list again
   const uint32_t raw = ((uint32_t*)e->h_pinned)[0];
   *raw_hits_out = raw;
   if (raw > hit_cap_now(e)) {
@@ -821,8 +885,11 @@ static int run_job_once(pps_engine* e, const pps_job_params* jp, pps_factor* out
   BaseTable bt;
   int rc = prepare_sieving_primes(e, jp->qmax, jp->pmax, &dq, &bt);
   if (rc) return rc;
-  CU(cudaMemsetAsync(e->counters.p, 0, 2 * sizeof(uint32_t), e->st));
+  CU(cudaMemsetAsync(e->counters.p, 0, CNT_WORDS * sizeof(uint32_t), e->st));
   int variant = -1;
+  TensorPlan plan;
+  const bool tensor = tensor_choice(e, jp, &plan);
+  if (tensor) variant = jp->sign == PPS_SIGN_TWIN ? VARIANT_TENSOR_TWIN : VARIANT_TENSOR;
   const uint64_t span = e->batch_span;
   for (uint64_t a = jp->pmin | 1ull; a < jp->pmax; a += span) {
     const uint64_t b = std::min(jp->pmax, a + span);
@@ -846,13 +913,17 @@ static int run_job_once(pps_engine* e, const pps_job_params* jp, pps_factor* out
     if (variant < 0) {
       variant = autotune(e, jp, e->P.p, e->Pinv.p, np);
       if (variant < 0) return variant;
-      if (st) st->variant = (uint32_t)variant;
     }
-    const int split = choose_split(e, jp, variant, np);
+    const int split = tensor ? (int)(TW_ROWS * plan.units) : choose_split(e, jp, variant, np);
     if (split < 0) return split;
-    if (st) st->split = std::max<uint32_t>(st->split, (uint32_t)split);
+    if (st) {
+      st->variant = (uint32_t)variant;
+      st->split = std::max<uint32_t>(st->split, (uint32_t)split);
+    }
     CU(cudaEventRecord(e->ev[2], e->st));
-    if ((rc = run_walk(e, jp, variant, e->P.p, e->Pinv.p, nullptr, np, 0, 0, (uint32_t)split))) return rc;
+    rc = tensor ? run_tensor_walk(e, jp, plan, e->P.p, e->Pinv.p, np)
+                : run_walk(e, jp, variant, e->P.p, e->Pinv.p, nullptr, np, 0, 0, (uint32_t)split);
+    if (rc) return rc;
     CU(cudaEventRecord(e->ev[3], e->st));
     if (st) {
       CU(cudaEventSynchronize(e->ev[3]));
@@ -900,10 +971,11 @@ extern "C" int pps_run_job(pps_engine* e, const pps_job_params* jp, pps_factor* 
   if (!e || !jp) return set_err(PPS_ERR_INVALID_PARAM, "null argument");
   if (jp->step < 1 || jp->step > 32 || jp->pmin <= (1ull << 32)) return set_err(PPS_ERR_INVALID_PARAM, "job not normalized");
   if (jp->sign == PPS_SIGN_TWIN) {
-    // twin jobs run on the batched walk, except with an input file: its rule
-    // applies on the one-job path, whose twin kernels need 32-bit steps or
-    // p <= 2^(32+s)
-    if (!e->input) return run_twin_job(e, jp, out, cap, nout, st);
+    // twin jobs run on the batched walk where the tensor walk is not faster,
+    // except with an input file: its rule applies on the one-job path, whose
+    // twin kernels need 32-bit steps or p <= 2^(32+s)
+    TensorPlan plan;
+    if (!e->input && !tensor_choice(e, jp, &plan)) return run_twin_job(e, jp, out, cap, nout, st);
     bool exact = false;
     for (int v = 0; v < PPS_NUM_VARIANTS && !exact; ++v) exact = variant_ok(jp, v) != 0;
     if (!exact)
@@ -937,17 +1009,30 @@ extern "C" int pps_run_job(pps_engine* e, const pps_job_params* jp, pps_factor* 
   return set_err(PPS_ERR_INSUFFICIENT_RESOURCE, "hit buffer overflow persisted");
 }
 
-// Walk primes already on the device; hits accumulate in e->hits.
+// Walk primes already on the device; hits accumulate in e->hits.  in_range: the
+// primes lie in [pmin, pmax), or the tensor walk, which needs that, has not
+// found otherwise yet.
 static int walk_device_list(pps_engine* e, const pps_job_params* jp, const uint64_t* dP, size_t np,
-                            pps_job_stats* st) {
-  int variant = autotune(e, jp, dP, nullptr, np);
+                            pps_job_stats* st, bool in_range) {
+  TensorPlan plan;
+  const bool tensor = in_range && tensor_choice(e, jp, &plan);
+  const int variant = !tensor ? autotune(e, jp, dP, nullptr, np)
+                              : jp->sign == PPS_SIGN_TWIN ? VARIANT_TENSOR_TWIN : VARIANT_TENSOR;
   if (variant < 0) return variant;
   if (st) st->variant = (uint32_t)variant;
-  const int split = choose_split(e, jp, variant, np);
+  const int split = tensor ? (int)(TW_ROWS * plan.units) : choose_split(e, jp, variant, np);
   if (split < 0) return split;
   if (st) st->split = (uint32_t)split;
   CU(cudaEventRecord(e->ev[2], e->st));
-  int rc = run_walk(e, jp, variant, dP, nullptr, nullptr, np, 0, 0, (uint32_t)split);
+  cudaPointerAttributes at;
+  if (tensor && cudaPointerGetAttributes(&at, dP) == cudaSuccess && at.type == cudaMemoryTypeHost) {
+    // a page-locked list: its re-check would read some primes a few times more
+    if (int rc = e->P.ensure(np)) return rc;
+    CU(cudaMemcpyAsync(e->P.p, dP, np * sizeof(uint64_t), cudaMemcpyDefault, e->st));
+    dP = e->P.p;
+  }
+  const int rc = tensor ? run_tensor_walk(e, jp, plan, dP, nullptr, np)
+                        : run_walk(e, jp, variant, dP, nullptr, nullptr, np, 0, 0, (uint32_t)split);
   if (rc) return rc;
   CU(cudaEventRecord(e->ev[3], e->st));
   if (st) {
@@ -968,17 +1053,23 @@ extern "C" int pps_check_primes_device(pps_engine* e, const pps_job_params* jp, 
   if (!e || !jp || (!d_P && np)) return set_err(PPS_ERR_INVALID_PARAM, "null argument");
   CU(cudaSetDevice(e->device));
   size_t hit_cap = 1u << 20, fac_cap = 1u << 18;
+  bool in_range = true;
   for (int attempt = 0; attempt < 4; ++attempt) {
     int rc = ensure_hit_buffers(e, std::max(hit_cap, e->hits.n), std::max(fac_cap, e->factors.n));
     if (rc) return rc;
     e->hit_cap_limit = attempt == 0 ? debug_first_hit_cap() : 0;
     if (st) memset(st, 0, sizeof *st);
-    CU(cudaMemsetAsync(e->counters.p, 0, 2 * sizeof(uint32_t), e->st));
-    if (np && (rc = walk_device_list(e, jp, d_P, np, st))) return rc;
-    bool overflow = false;
+    CU(cudaMemsetAsync(e->counters.p, 0, CNT_WORDS * sizeof(uint32_t), e->st));
+    if (np && (rc = walk_device_list(e, jp, d_P, np, st, in_range))) return rc;
+    bool overflow = false, outside = false;
     uint32_t raw = 0;
-    rc = finish_job(e, jp, out, cap, nout, st, &raw, &overflow);
+    rc = finish_job(e, jp, out, cap, nout, st, &raw, &overflow, &outside);
     if (st) st->raw_hits = raw;
+    if (!rc && outside) {  // not an attempt: the list is walked by the recurrence from here on
+      in_range = false;
+      --attempt;
+      continue;
+    }
     if (rc || !overflow) return rc;
     // grow the buffers, unless the overflow was only the first attempt's
     // debug cap (the retry lifts it)
@@ -1035,13 +1126,21 @@ extern "C" int pps_check_primes_raw(pps_engine* e, const pps_job_params* jp, con
   const uint64_t* dP;
   if ((rc = host_list_on_device(e, P, np, &dP))) return rc;
   size_t hit_cap = std::max<size_t>(1u << 20, e->hits.n);
+  bool in_range = true;
   for (int attempt = 0; attempt < 4; ++attempt) {
     if ((rc = ensure_hit_buffers(e, hit_cap, std::max<size_t>(1u << 18, e->factors.n)))) return rc;
     e->hit_cap_limit = attempt == 0 ? debug_first_hit_cap() : 0;
-    CU(cudaMemsetAsync(e->counters.p, 0, 2 * sizeof(uint32_t), e->st));
-    if (np && (rc = walk_device_list(e, jp, dP, np, nullptr))) return rc;
-    CU(cudaMemcpyAsync(e->h_pinned, e->counters.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, e->st));
+    CU(cudaMemsetAsync(e->counters.p, 0, CNT_WORDS * sizeof(uint32_t), e->st));
+    if (np && (rc = walk_device_list(e, jp, dP, np, nullptr, in_range))) return rc;
+    CU(cudaMemcpyAsync(e->h_pinned, e->counters.p, CNT_WORDS * sizeof(uint32_t), cudaMemcpyDeviceToHost, e->st));
     CU(cudaStreamSynchronize(e->st));
+    bool outside = false;
+    if ((rc = tensor_status(e, &outside))) return rc;
+    if (outside) {  // not an attempt: the list is walked by the recurrence from here on
+      in_range = false;
+      --attempt;
+      continue;
+    }
     const uint32_t raw = ((uint32_t*)e->h_pinned)[0];
     if (raw > hit_cap_now(e)) {
       hit_cap = std::max<size_t>(hit_cap, raw > e->hits.n ? (size_t)raw * 2 : e->hits.n);

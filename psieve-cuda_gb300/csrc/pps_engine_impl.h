@@ -63,6 +63,8 @@ struct DevBuf {
   size_t bytes() const { return n * sizeof(T); }
 };
 
+constexpr uint32_t CNT_TENSOR = 4, CNT_WORDS = 8;  // words of pps_engine::counters
+
 struct BatchState;  // pps_batch.cu
 
 struct pps_engine {
@@ -108,12 +110,13 @@ struct pps_engine {
   DevBuf<uint64_t> totals;  // [0] count, [1] sum
   DevBuf<pps_hit> hits;
   DevBuf<pps_factor> factors;
-  DevBuf<uint32_t> counters;  // [0] raw hits, [1] factors
+  DevBuf<uint32_t> counters;  // [0] raw hits, [1] factors, [CNT_TENSOR..] the tensor walk's work and status words
   DevBuf<uint16_t> small_q;
   DevBuf<uint32_t> presieve;  // the pre-sieve table for 3, 5, 7, 11, 13 (PRESIEVE_WORDS)
   DevBuf<uint32_t> sieve_res; // per-batch residues of the small sieving primes
   uint32_t nsmall = 0;
   DevBuf<uint32_t> probe_sink;
+  DevBuf<uint4> masks;        // the tensor walk's passing rows
   uint64_t* h_pinned = nullptr;  // 16 words of pinned host scratch
 
   BatchState* batch = nullptr;  // state of the batched persistent form

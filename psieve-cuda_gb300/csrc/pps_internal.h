@@ -109,7 +109,9 @@ struct VariantTraits {
   bool stepwin;
   int unroll;      // steps per block
   int per_thread;  // primes per thread (queued walks: a warp covers 32 x this)
+  bool tensor;     // the tensor walk (pps_tensor.cu); the rest does not apply but `twin`
 };
+constexpr int VARIANT_TENSOR = 31, VARIANT_TENSOR_TWIN = 32;
 const VariantTraits& walk_variant_traits(int v);
 // Pre-test constants of a normalised job, and whether variant v is exact for it
 // (defined in pps_engine.cu).

@@ -725,7 +725,7 @@ __global__ void __launch_bounds__(256, MINB) k_walk32q2(WalkArgs a) {
   }
 }
 
-// name, queued, twin, s32, shifted, smallp, min_window, bound, lowbit, stepwin, unroll, per_thread
+// name, queued, twin, s32, shifted, smallp, min_window, bound, lowbit, stepwin, unroll, per_thread, tensor
 static const VariantTraits kVariants[PPS_NUM_VARIANTS] = {
     {"form0-window-u4-step", false, false, false, false, false, false, false, false, false, 4, 1},
     {"chain-window-u4-step", false, false, false, false, false, false, false, false, false, 4, 1},
@@ -758,6 +758,8 @@ static const VariantTraits kVariants[PPS_NUM_VARIANTS] = {
     {"queue-min-u16-r40", true, false, true, false, false, true, false, false, false, 16, 1},
     {"queue-bound-u16-r40", true, false, true, false, false, false, true, false, false, 16, 1},
     {"queue2-bound-u16", true, false, true, false, false, false, true, false, false, 16, 2},
+    {"tensor", false, false, false, false, false, false, false, false, false, 1, 1, true},
+    {"twin-tensor", false, true, false, false, false, false, false, false, false, 1, 1, true},
 };
 
 const VariantTraits& walk_variant_traits(int v) {

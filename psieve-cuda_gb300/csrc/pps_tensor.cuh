@@ -1,0 +1,57 @@
+// pps_tensor.cuh -- the tensor walk: plan, arguments and launcher shared by the
+// one-job and batched host code.  The kernel is in pps_tensor.cu.
+#pragma once
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include "pps_internal.h"
+
+namespace pps {
+
+constexpr uint32_t TW_ROWS = 128;    // MMA rows: giant steps of one unit
+constexpr uint32_t TW_MAX_NB = 512;  // columns (baby steps) of one unit, at most
+
+// How one job runs on the tensor walk (tensor_plan).
+struct TensorPlan {
+  uint32_t s;       // n per test
+  uint32_t nb;      // columns: tests per row, a multiple of 16
+  uint32_t units;   // units of 128 x nb tests per prime
+  uint32_t digits;  // bits per digit: 4 (p < 2^47) or 5 (p < 2^62)
+  uint32_t pitch;   // words of a prime's expansion in shared memory (odd)
+  uint32_t off;     // offset of the tested fraction, and the test's bound, in 2^-16
+  uint32_t thr;
+  double cost;      // estimated SM clocks per prime
+};
+
+// Whether the tensor walk can run the job at all, and how.
+bool tensor_plan(const pps_job_params* jp, TensorPlan* out);
+
+struct TensorArgs {
+  const uint64_t* P;
+  const uint64_t* Pinv;  // or null: computed
+  uint64_t np;
+  uint64_t pmin, pmax, kmin, kmax;
+  uint32_t nmin, nmax;
+  uint32_t side;         // 1: K = -2^-n (Proth), 0: K = 2^-n (Riesel), 2: both (twin)
+  uint32_t idx_base;
+  TensorPlan plan;
+  uint32_t batch;        // units a CTA takes at a time (1..32)
+  uint32_t* work;        // [0] batches taken (zeroed before each launch)
+                         // [1] set when a prime outside [pmin, pmax) was met (not walked)
+                         // [2] set when a bounded wait ran out
+  uint4* masks;          // which rows pass: of each unit, tile and 32 rows a bit per row for columns 0-31,
+                         // 32-63, 64-95 and 96-111 of the tile
+  pps_hit* hits;
+  uint32_t* hit_count;
+  uint32_t hit_cap;
+};
+
+constexpr double TW_LEAST_COST = 710.0;      // of one unit (TensorPlan::cost)
+constexpr uint32_t TW_MAX_MASKS = 1u << 24;  // 268 MB; their numbers have 25 bits in k_tensor_check
+
+// Masks for np primes, or for one part of them.
+size_t tensor_masks(const TensorPlan& plan, uint64_t np);
+// The walk and the re-check of np primes, in parts of TW_MAX_MASKS masks.  *launches += the kernels launched.
+cudaError_t launch_tensor_walk(TensorArgs a, int num_sms, cudaStream_t st, uint64_t* launches);
+
+}  // namespace pps

@@ -31,8 +31,8 @@ PPS_ERR_TIMEOUT = -303
 PPS_ERR_BUSY = -304
 PPS_ERR_NOT_FOUND = -305
 PPS_ERR_CANCELLED = -306
-PPS_NUM_VARIANTS = 31
-TWIN_VARIANTS = (22, 23, 24, 25)  # the walks of both sides of a twin job
+PPS_NUM_VARIANTS = 33
+TWIN_VARIANTS = (22, 23, 24, 25, 32)  # the walks of both sides of a twin job
 PPS_SIGN_TWIN = 2  # both sides from one walk (the reference's twin build)
 PPS_NOALLOC_MAX_PRIMES = 1 << 24  # per call of pps_check_primes_noalloc
 PPS_NOALLOC_MAX_CANDIDATES = 1 << 16
@@ -283,6 +283,8 @@ def walk_variant_name(v: int, lib=None) -> str:
 def walk_kernel_name(v: int, lib=None) -> str:
     """The CUDA kernel that runs walk variant v."""
     name = walk_variant_name(v, lib)
+    if name.endswith("tensor"):
+        return "k_tensor_walk"
     if name.startswith("queue2"):
         return "k_walk32q2"
     if name.startswith(("queue", "twin")):
