@@ -696,13 +696,13 @@ static int autotune(pps_engine* e, const pps_job_params* jp, const uint64_t* dP,
 
 // Whether the job runs on the tensor walk, and how: where its cost is estimated
 // to be below the recurrence's, both in SM clocks per prime.  tensor_plan's
-// estimate holds within 8%.  The recurrence's is its steps times what one took
+// estimate holds within 9%.  The recurrence's is its steps times what one took
 // with 1.5 to 2.4 million primes: 32-bit steps 0.106-0.110 (p up to 2^50;
 // 0.089 at 2^62), shorter ones 0.135, a twin step 0.19-0.24 (on the batched
-// form).  On either side of the line: p = 4.2e13, N = 200,000: 693 clocks
-// against the tensor walk's 793, N = 300,000: 1,032 against 915; p = 2^62, N =
-// 300,000: 852 against 903, N = 600,000: 1,685 against 1,337; p = 10^12, N =
-// 150,000: 764 against 797, N = 200,000: 1,012 against 826.
+// form).  On either side of the line: p = 4.2e13, N = 200,000: 692 clocks
+// against the tensor walk's 714, N = 250,000: 861 against 740; p = 2^62, N =
+// 250,000: 711 against 761, N = 300,000: 852 against 784; p = 10^12, N =
+// 131,071: 669 against 713, N = 150,000: 764 against 724.
 static bool tensor_choice(const pps_engine* e, const pps_job_params* jp, TensorPlan* plan) {
   const bool twin = jp->sign == PPS_SIGN_TWIN;
   const int v = twin ? VARIANT_TENSOR_TWIN : VARIANT_TENSOR;

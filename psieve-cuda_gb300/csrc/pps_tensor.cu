@@ -35,7 +35,7 @@
 // One CTA per SM, its warps in roles (mbarriers between them):
 //   2 seed warps    batch of 32 units, lane = unit: the expansion S, the
 //                   tables c^j (16) and K_0 c^16i (8), c = 2^-(s nb)
-//   8 build warps   two groups, unit by unit: A rows (thread = row) into TMEM,
+//   12 build warps  three groups, unit by unit: A rows (thread = row) into TMEM,
 //                   B rows into shared memory
 //   2 MMA warps     one to each half of the accumulators: two tiles of 112
 //                   columns at a time (a wait and the two MMAs after it take a
@@ -45,15 +45,19 @@
 //                   pass in each 32 columns: a mask to global memory
 // and a second kernel, one thread to a passing row.
 //
-// Measured, 8.56 million primes at 4.2e13, a million n: 41.7 ms, of which the
+// Measured, 8.56 million primes at 4.2e13, a million n: 40.2 ms, of which the
 // second kernel 12%, against 91.0 ms of the recurrence; 6.24 million at 2^62,
-// 900,000 n: 26.7 against 47.9 ms.  What bounds the first kernel is the issue
-// of instructions (70% of the slots, the integer pipe 72% busy), no longer
-// multiplies: about 90 a warp and test tile, of them 32 the minima, 45 a B row
-// warp, 200 an A warp.  The MMAs fill 224 of the 1,350 clocks of a prime.
+// 900,000 n: 23.5 against 47.9 ms.  What bounds the first kernel is the issue
+// of instructions (3,460 a prime, 71% of the slots, the integer pipe 73% busy),
+// no longer multiplies: about 90 a warp and test tile, of them 32 the minima,
+// 50 a B row warp, 200 an A warp.  Its chains come close behind: the build warps
+// spend 60% of a prime's 1,300 clocks on their rows (a third group took the
+// cases above from 41.7 and 26.7 ms), a test warp 70% on its tile.  The MMAs
+// fill 224 clocks.  A tile in one load, which frees it sooner but holds 24
+// registers more, made no difference.
 // Passing rows that the test warps re-check themselves, or hand over with their
 // fractions, hold up all eight warps of a half (2,450 and 2,114 clocks a prime
-// with everything else as it was); so they only store a mask.
+// where a mask took 1,838); so they only store a mask.
 //
 // Reference counterpart: the walk of pps/appcu.cu:779-1190 (one 32-n step per
 // three multiplies); the candidates are the same set.
@@ -72,10 +76,13 @@ namespace pps {
 
 namespace {
 
-constexpr uint32_t TW_GROUPS = 4, TW_BGROUPS = 2;  // test and build groups of four warps
+constexpr uint32_t TW_GROUPS = 4, TW_BGROUPS = 3;  // test and build groups of four warps
 constexpr int TW_TEST_WARPS = 4 * TW_GROUPS, TW_BUILD_WARPS = 4 * TW_BGROUPS, TW_SEED_WARPS = 2, TW_MMA_WARPS = 2;
 constexpr int TW_THREADS = 32 * (TW_TEST_WARPS + TW_BUILD_WARPS + TW_SEED_WARPS + TW_MMA_WARPS);
-constexpr uint32_t TW_STAGES = 4;   // A and B operand stages
+constexpr uint32_t TW_STAGES = 3;   // A and B operand stages
+// A waiter of a barrier has to see each of its phases (it tells only odd from
+// even): a build group keeps to its stages, and both MMA warps wait for every unit.
+static_assert(TW_STAGES % TW_BGROUPS == 0, "a stage belongs to one build group");
 constexpr uint32_t TW_TILE = 112;   // columns of one tile
 constexpr uint32_t TW_PART = 32;    // and of one word of a tile's masks
 constexpr uint32_t TW_ACOL = TW_GROUPS * TW_TILE;  // first TMEM column of the A stages (16 each)
@@ -338,7 +345,7 @@ __device__ __forceinline__ uint32_t min16(const uint32_t* q) {
 
 // ---- the kernel
 
-// G: bits per digit.  896 threads, at most 72 registers each.
+// G: bits per digit.  1,024 threads, at most 64 registers each.
 template <int G>
 __global__ void __launch_bounds__(TW_THREADS, 1) k_tensor_walk(const __grid_constant__ TensorArgs a) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
@@ -357,7 +364,7 @@ __global__ void __launch_bounds__(TW_THREADS, 1) k_tensor_walk(const __grid_cons
     }
     for (uint32_t i = 0; i < TW_STAGES; ++i) {
       mbar_init(smem_addr(&sh->ab_full[i]), 4);
-      mbar_init(smem_addr(&sh->ab_empty[i]), npairs > 1u ? 2u : 1u);
+      mbar_init(smem_addr(&sh->ab_empty[i]), TW_MMA_WARPS);
     }
     for (uint32_t i = 0; i < TW_GROUPS; ++i) {
       mbar_init(smem_addr(&sh->d_full[i]), 1);
@@ -403,24 +410,24 @@ __global__ void __launch_bounds__(TW_THREADS, 1) k_tensor_walk(const __grid_cons
           if (!(ok = mbar_wait<0>(full, par, give_up))) break;
           par ^= 1u;
           tc_fence_after();
-          uint32_t q[56];
-          tmem_ld112_lo16(q, src);
+          uint32_t q[32], m[4];
+          auto passing = [&](uint32_t v) { return __ballot_sync(0xffffffffu, min(v, v << 16) < thr16); };
+          // G == 5: a fraction of 15 bits below one whole bit; the pair shifted left
+          // drops it (a bit moves into the upper fraction's last place)
+          tmem_ld64_lo16(q, src);
+#pragma unroll
+          for (int i = 0; i < 32; ++i) q[i] += G == 5 ? q[i] : 0u;
+          m[0] = passing(min16(q));
+          m[1] = passing(min16(q + 16));
+          tmem_ld48_lo16(q, src + 64u);
           tc_fence_before();
           __syncwarp();
           // (a pair's only tile arrives for both)
           mbar_arrive_lane0(empty, (group & 1u) == 0u && t + 1u == ntiles ? 2u : 1u);
-          if (G == 5) {
-            // fraction of 15 bits below one whole bit: the pair shifted left drops
-            // it (a bit moves into the upper fraction's last place)
 #pragma unroll
-            for (int i = 0; i < 56; ++i) q[i] += q[i];
-          }
-          uint32_t m[4];
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const uint32_t v = i < 3 ? min16(q + 16 * i) : min8(q + 48);
-            m[i] = __ballot_sync(0xffffffffu, min(v, v << 16) < thr16);
-          }
+          for (int i = 0; i < 24; ++i) q[i] += G == 5 ? q[i] : 0u;
+          m[2] = passing(min16(q));
+          m[3] = passing(min8(q + 16));
           if (lane == 0) out[t * 4u] = make_uint4(m[0], m[1], m[2], m[3]);
         }
         skip -= npairs;
@@ -484,7 +491,6 @@ __global__ void __launch_bounds__(TW_THREADS, 1) k_tensor_walk(const __grid_cons
     constexpr uint32_t OFF = G == 4 ? 64u : 96u;
     const uint64_t nunits = a.np * a.plan.units;
     const uint32_t words = ((s * (nb - 1u)) >> 5) + (G == 4 ? 3u : 4u);  // read by b_row
-    const uint32_t half = words / 2u;
     const uint32_t stride = s * nb;  // n between rows
     bool ok = true;
     for (uint32_t it = 0; ok; ++it) {
@@ -513,42 +519,48 @@ __global__ void __launch_bounds__(TW_THREADS, 1) k_tensor_walk(const __grid_cons
         }
         uint64_t* tab = sh->tab[slot][lane];
         {
-          // the expansion: words [0, half) from K = 1, the rest from 2^-(32 half)
+          // the expansion, a quarter of its words from each of the starts 2^-(32 w), two
+          // quarters to a warp: independent chains that fill each other's latencies
           uint32_t* Sp = S + ((size_t)slot * 32u + lane) * pitch;
-          const uint32_t w0 = part ? half : 0u, w1 = part ? words : half;
-          const uint64_t K = part && half ? inv_pow2(32u * half, p, ps) : 1ull;
-          uint32_t klo = lo32(K), khi = hi32(K);
+          const uint32_t quarter = (words + 3u) >> 2, w0 = 2u * part * quarter;
+          const uint64_t K = w0 ? inv_pow2(32u * w0, p, ps) : 1ull, K2 = inv_pow2(32u * (w0 + quarter), p, ps);
+          uint32_t klo = lo32(K), khi = hi32(K), klo2 = lo32(K2), khi2 = hi32(K2);
           const uint32_t plon = neg_lo(p), phi1 = neg_hi(p), pinv = lo32(ps);
-          for (uint32_t w = w0; w < w1; ++w) {
-            const uint32_t m = klo * pinv;
+          for (uint32_t w = w0; w < w0 + quarter; ++w) {
+            const uint32_t m = klo * pinv, m2 = klo2 * pinv;
             Sp[w] = m;
+            Sp[w + quarter] = m2;  // (the pitch holds four quarters)
             neg_sum(m, khi, plon, phi1, klo, khi);
+            neg_sum(m2, khi2, plon, phi1, klo2, khi2);
           }
         }
+        // the tables, every second value from each of two starts
         if (part == 0u) {
           // H_j = c^j 2^64 mod p, c = 2^-stride
-          uint64_t h = (0ull - p) % p;
-          const uint64_t c = inv_pow2(stride - 64u, p, ps);
+          uint64_t h = (0ull - p) % p, h2 = inv_pow2(stride - 64u, p, ps);
+          const uint64_t c2 = mont_mul(h2, h2, p, ps);
           tab[TAB_P] = p;
           tab[TAB_PS] = ps;
-          tab[TAB_H] = h;
-          h = c;
 #pragma unroll 1
-          for (uint32_t j = 1;; ++j) {
+          for (uint32_t j = 0;; j += 2u) {
             tab[TAB_H + j] = h;
-            if (j == 15u) break;
-            h = mont_mul(h, c, p, ps);
+            tab[TAB_H + j + 1u] = h2;
+            if (j == 14u) break;
+            h = mont_mul(h, c2, p, ps);
+            h2 = mont_mul(h2, c2, p, ps);
           }
         } else {
           // G_i = K_0 c^(16 i); c^16 in Montgomery form
           const uint64_t x = inv_pow2(a.nmin + stride * TW_ROWS * ta - OFF, p, ps);
-          uint64_t g = a.side == 1u ? p - x : x;
-          const uint64_t c16 = inv_pow2(16u * stride - 64u, p, ps);
+          const uint64_t c16 = inv_pow2(16u * stride - 64u, p, ps), c32 = mont_mul(c16, c16, p, ps);
+          uint64_t g = a.side == 1u ? p - x : x, g2 = mont_mul(g, c16, p, ps);
 #pragma unroll 1
-          for (uint32_t i = 0;; ++i) {
+          for (uint32_t i = 0;; i += 2u) {
             tab[i] = g;
-            if (i == 7u) break;
-            g = mont_mul(g, c16, p, ps);
+            tab[i + 1u] = g2;
+            if (i == 6u) break;
+            g = mont_mul(g, c32, p, ps);
+            g2 = mont_mul(g2, c32, p, ps);
           }
         }
       }
@@ -573,10 +585,11 @@ __global__ void __launch_bounds__(TW_THREADS, 1) k_tensor_walk(const __grid_cons
       if (!count) break;
       // this half's pairs of the batch's units, in order
       for (uint32_t unit = 0; unit < count && ok; ++unit, ++unit_no) {
-        if (skip < npairs) {
-          const uint32_t st = unit_no % TW_STAGES;
-          if (!(ok = mbar_wait<0>(abf0 + st * 8u, (unit_no / TW_STAGES) & 1u, give_up))) break;
-          const uint32_t atm = TW_ACOL + st * 16u, b_st = b_lo + st * nbp * 2u;
+        const uint32_t st = unit_no % TW_STAGES;
+        if (!(ok = mbar_wait<0>(abf0 + st * 8u, (unit_no / TW_STAGES) & 1u, give_up))) break;
+        const uint32_t atm = TW_ACOL + st * 16u, b_st = b_lo + st * nbp * 2u;
+        if (skip >= npairs) mbar_arrive_lane0(abe0 + st * 8u);  // a unit of one pair, the other half's
+        else {
           for (; skip < npairs; skip += 2u) {
             if (!(ok = mbar_wait<0>(empty, free_par, give_up))) break;
             free_par ^= 1u;
@@ -611,8 +624,8 @@ size_t tensor_smem(uint32_t nb, uint32_t pitch) {
 
 // For each number of units the columns and the stride that cover the n range,
 // by an estimate of the SM clocks per prime: set-up and A rows per unit, B rows
-// and tests per column and tile, and the re-check of what passes.  Fitted to 20
-// sizes from 30,000 to 4 million n at p = 10^12 to 2^62, within 8% of each.
+// and tests per column and tile, and the re-check of what passes.  Fitted to 48
+// sizes from 30,000 to 2 million n at p = 10^12 to 2^62, within 9% of each.
 bool tensor_plan(const pps_job_params* jp, TensorPlan* out) {
   if (jp->nmax <= jp->nmin || jp->nmin < 128u || jp->pmin <= (1ull << 32) || jp->pmax > (1ull << 62)) return false;
   if (jp->pmax <= jp->pmin || jp->kmax < jp->kmin) return false;
@@ -630,7 +643,8 @@ bool tensor_plan(const pps_job_params* jp, TensorPlan* out) {
       if (s > 60 || s * nb < 128) continue;
       const double eps = one * ldexp(1.0, (int)s - 1);
       if (eps > 1000.0) continue;
-      const uint32_t pitch = (uint32_t)((((s * (nb - 1)) >> 5) + (g == 4u ? 3u : 4u)) | 1u);
+      // the words that b_row reads, in four quarters, and odd: 32 units' words lie in 32 banks
+      const uint32_t words = (uint32_t)((s * (nb - 1)) >> 5) + (g == 4u ? 3u : 4u), pitch = ((words + 3u) & ~3u) + 1u;
       if (tensor_smem(nb, pitch) > TW_MAX_SMEM) continue;
       const bool twin = jp->sign == PPS_SIGN_TWIN;
       TensorPlan t;
@@ -643,7 +657,7 @@ bool tensor_plan(const pps_job_params* jp, TensorPlan* out) {
       t.thr = t.off + (uint32_t)floor(eps + above) + 1u;
       const double passes = (double)TW_ROWS * nb * t.thr / 65536.0;
       const double tiles = (double)((nb + TW_TILE - 1) / TW_TILE);
-      t.cost = (double)units * ((g == 4u ? 560.0 + 150.0 * tiles : 670.0 + 190.0 * tiles) + 0.43 * nb + 33.0 * passes);
+      t.cost = (double)units * (460.0 + (g == 4u ? 175.0 : 225.0) * tiles + 0.43 * nb + 33.0 * passes);
       if (!found || t.cost < out->cost) {
         *out = t;
         found = true;

@@ -46,7 +46,7 @@ struct TensorArgs {
   uint32_t hit_cap;
 };
 
-constexpr double TW_LEAST_COST = 710.0;      // of one unit (TensorPlan::cost)
+constexpr double TW_LEAST_COST = 635.0;      // of one unit (TensorPlan::cost)
 constexpr uint32_t TW_MAX_MASKS = 1u << 24;  // 268 MB; their numbers have 25 bits in k_tensor_check
 
 // Masks for np primes, or for one part of them.
