@@ -11,22 +11,27 @@
 // chunks of CHUNK primes (all of one job, so every lane of a warp has the same
 // n loop) from a device counter until the wave is exhausted.  Raw candidates
 // carry their job slot; a filter launch after each wave applies each job's
-// output rule.  Jobs live in device slots (parameters, prime counters), so the
+// output rule.  A job with a long n range has no chunks: the tensor walk takes
+// its primes in launches of its own after the walk kernel, from offsets that the
+// host reads while that runs.  Jobs live in device slots (parameters, prime counters), so the
 // serving loop can admit and retire jobs between waves.
 //
 // Reference counterpart: none in one piece -- the reference runs one range per
 // process (main.c:887-1266) and one kernel per n slice (pps/appcu.cu:1194-1261).
 #include <cuda_runtime.h>
+#include <math.h>
 #include <stddef.h>
 #include <stdio.h>
 #include <string.h>
 
 #include <algorithm>
+#include <unordered_map>
 #include <vector>
 
 #include "pps_device.cuh"
 #include "pps_engine_impl.h"
 #include "pps_sieve.cuh"
+#include "pps_tensor.cuh"
 
 namespace pps {
 
@@ -59,6 +64,13 @@ struct BJob {
   // L = ceil(blocks / nsplit), so a long-n job's work comes in pieces of
   // about the same size as a short-n job's
   uint32_t nsplit;
+  uint32_t tensor;  // walked by the tensor walk (no chunks)
+};
+
+// A slot's job that the tensor walk takes.
+struct TensorSlot {
+  pps_job_params job;
+  TensorPlan plan;
 };
 
 struct BBatch {
@@ -114,6 +126,9 @@ struct BatchState {
   int tuned_work = 0, tuned_unroll = 0;  // walk steps per chunk (x32 lanes), walk kernel code (timed)
   int walk_code = 0;                     // the walk kernel code of the last wave (tuned or forced)
   std::vector<BJob> hjobs;               // host mirror of the device job slots
+  std::unordered_map<uint32_t, TensorSlot> tensor;  // the slots that the tensor walk takes
+  uint32_t* h_off = nullptr;             // pinned: each segment's first prime in P, and the end
+  int wave_work = 0;                     // walk steps per chunk of the last wave
   std::vector<uint64_t> slot_pmax;       // each slot's pmax (sieving-prime bound)
   DevBuf<unsigned long long> bak_primes, bak_sum;  // slot counters before a wave
 };
@@ -133,6 +148,7 @@ void batch_state_free(pps_engine* e) {
     if (v) cudaEventDestroy(v);
   if (b->copied) cudaEventDestroy(b->copied);
   if (b->h_tables) cudaFreeHost(b->h_tables);
+  if (b->h_off) cudaFreeHost(b->h_off);
   b->tables.release();
   b->jobs.release();
   b->bitmap.release();
@@ -420,7 +436,7 @@ __global__ void k_bchunks(const uint8_t* tables, const BJob* jobs, const uint32_
     uint32_t n = 0;
     if (s < T->nseg) {
       const BJob& J = jobs[T->batch[T->seg[s].batch].job];
-      n = (seg_count[s] + J.chunk - 1) / J.chunk * J.nsplit;
+      n = J.tensor ? 0u : (seg_count[s] + J.chunk - 1) / J.chunk * J.nsplit;
     }
     chunk_count[s] = n;
   }
@@ -866,6 +882,10 @@ int ensure_state(pps_engine* e) {
       b->h_tables = nullptr;
       return set_err(PPS_ERR_INSUFFICIENT_RESOURCE, "pinned table staging");
     }
+    if (!b->h_off && cudaMallocHost(&b->h_off, (WAVE_SEGS + 2) * sizeof(uint32_t)) != cudaSuccess) {
+      b->h_off = nullptr;
+      return set_err(PPS_ERR_INSUFFICIENT_RESOURCE, "pinned segment offsets");
+    }
     b->wave_segs = e->wave_segs_req ? e->wave_segs_req : WAVE_SEGS;
     if ((rc = b->bitmap.ensure((size_t)b->wave_segs * SEG_WORDS))) return rc;
     if ((rc = b->seg_count.ensure(WAVE_SEGS)) || (rc = b->seg_off.ensure(WAVE_SEGS)) ||
@@ -964,6 +984,28 @@ int launch_wave(pps_engine* e, const uint32_t* dq, uint32_t nq_all, int unroll, 
                 pps_hit* hits, uint32_t* hit_count, uint32_t hit_cap) {
   int rc = launch_wave_sieve(e, dq, nq_all);
   return rc ? rc : launch_wave_walk(e, unroll, chunk_limit, hits, hit_count, hit_cap);
+}
+
+// The wave's jobs that the tensor walk takes: the primes of each one's batches
+// that follow each other.  The host reads the segments' offsets while the
+// others are walked.
+int launch_wave_tensor(pps_engine* e, const WaveTables* T, uint32_t hit_cap) {
+  BatchState* b = e->batch;
+  CU(cudaMemsetAsync(e->counters.p + CNT_TENSOR, 0, (CNT_WORDS - CNT_TENSOR) * sizeof(uint32_t), e->st));
+  CU(cudaEventSynchronize(b->ev_wave[1]));
+  for (uint32_t i = 0, z; i < T->nbatch; i = z) {
+    const uint32_t slot = T->batch[i].job;
+    for (z = i + 1; z < T->nbatch && T->batch[z].job == slot;) ++z;
+    const auto t = b->tensor.find(slot);
+    if (t == b->tensor.end()) continue;
+    const uint32_t p0 = b->h_off[T->batch[i].seg0], p1 = b->h_off[z < T->nbatch ? T->batch[z].seg0 : T->nseg];
+    if (p1 == p0) continue;
+    const uint32_t idx = slot | (t->second.job.sign == 1 ? SIDE_PROTH : 0u);
+    if (int rc = run_tensor_walk(e, &t->second.job, t->second.plan, b->P.p + p0, b->Pinv.p + p0, p1 - p0,
+                                 TensorHits{b->hits.p, b->counters.p, hit_cap, idx, 0u}))
+      return rc;
+  }
+  return PPS_OK;
 }
 
 int floor_lg2(uint64_t x) { return 63 - __builtin_clzll(x | 1ull); }
@@ -1114,6 +1156,11 @@ void batch_tuning(pps_engine* e, uint32_t* work, uint32_t* unroll) {
   if (unroll) *unroll = b ? (uint32_t)b->walk_code & 0xffu : 0;
 }
 
+// A job leaves the walk kernel for launches of its own where the tensor walk
+// saves more SM clocks than those cost (two kernels and their tails, about 30 us
+// of 152 SMs).
+constexpr double TENSOR_LEAST_SAVED = 1e7;
+
 int batch_set_jobs(pps_engine* e, uint32_t slot0, const pps_job_params* jobs, size_t n) {
   int rc;
   if ((rc = batch_prepare(e))) return rc;
@@ -1127,6 +1174,15 @@ int batch_set_jobs(pps_engine* e, uint32_t slot0, const pps_job_params* jobs, si
   for (size_t j = 0; j < n; ++j) {
     BJob J = make_job(jobs[j]);
     chunk_for(&J, work, e->forced_split);
+    TensorSlot t;
+    double saved = 0;
+    b->tensor.erase((uint32_t)(slot0 + j));
+    if (!e->forced_bwalk && tensor_choice(e, &jobs[j], &t.plan, &saved) &&
+        saved * (double)(jobs[j].pmax - jobs[j].pmin) > TENSOR_LEAST_SAVED * log((double)jobs[j].pmin)) {
+      t.job = jobs[j];
+      J.tensor = 1;
+      b->tensor[(uint32_t)(slot0 + j)] = t;
+    }
     b->hjobs[slot0 + j] = J;
     b->slot_pmax[slot0 + j] = jobs[j].pmax;
   }
@@ -1239,7 +1295,15 @@ int batch_wave(pps_engine* e, const BatchPiece* pieces, size_t n, std::vector<pp
     return PPS_OK;
   };
 
-  if (!b->tuned_work) {
+  // the tensor walk's jobs, and the first batch of the others
+  bool tensor = false;
+  uint32_t first = nb;
+  for (uint32_t i = 0; i < nb; ++i) {
+    const bool t = b->hjobs[T->batch[i].job].tensor != 0;
+    tensor = tensor || t;
+    if (!t && first == nb) first = i;
+  }
+  if (!b->tuned_work && first < nb) {
     // time each (work per chunk, unroll) on the first chunks of this wave, the
     // same number of walk steps for every candidate.  The kernels take two
     // primes per lane: on the 512-job mix, each kind of job alone walked as
@@ -1272,11 +1336,11 @@ int batch_wave(pps_engine* e, const BatchPiece* pieces, size_t n, std::vector<pp
         float ms = 0;
         CU(cudaEventElapsedTime(&ms, e->ev[0], e->ev[1]));
         // steps timed: the work items walked (the wave may hold fewer than lim),
-        // each with the chunk size and n part of the wave's first job, whose
-        // primes come first
+        // each with the chunk size and n part of the first job they belong to,
+        // whose primes come first
         uint64_t nch = 0;
         CU(cudaMemcpy(&nch, b->tot.p + 2, sizeof nch, cudaMemcpyDeviceToHost));
-        const BJob& J0 = b->hjobs[T->batch[0].job];
+        const BJob& J0 = b->hjobs[T->batch[first].job];
         const double part_steps = (double)std::max<uint32_t>(J0.nsteps, 1) / std::max<uint32_t>(J0.nsplit, 1);
         const double steps = (double)std::min<uint64_t>(lim, nch) * J0.chunk * part_steps;
         const float per_step = (float)(ms / std::max(steps, 1.0));
@@ -1289,8 +1353,10 @@ int batch_wave(pps_engine* e, const BatchPiece* pieces, size_t n, std::vector<pp
     if ((rc = restore())) return rc;
   }
   // the walk kernel of this wave: the tuner's, unless pps_engine_set_batch_walk forces one
-  b->walk_code = e->forced_bwalk ? e->forced_bwalk : b->tuned_unroll;
-  if ((rc = set_chunks(e, smin, smax, b->tuned_work))) return rc;
+  // (a first wave of the tensor walk's jobs alone has timed nothing)
+  b->walk_code = e->forced_bwalk ? e->forced_bwalk : b->tuned_unroll ? b->tuned_unroll : 8 | WALK_TWO;
+  b->wave_work = b->tuned_work ? b->tuned_work : 1024;
+  if ((rc = set_chunks(e, smin, smax, b->wave_work))) return rc;
 
   // the wave itself: a captured graph of the fixed sequence, replayed
   CU(cudaMemsetAsync(b->counters.p, 0, 2 * sizeof(uint32_t), st));
@@ -1328,12 +1394,25 @@ int batch_wave(pps_engine* e, const BatchPiece* pieces, size_t n, std::vector<pp
     }
     CU(cudaEventRecord(b->ev_wave[0], st));
     CU(cudaGraphLaunch(b->graph, st));
+    if (tensor) {
+      CU(cudaMemcpyAsync(b->h_off, b->seg_off.p, nseg * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+      CU(cudaMemcpyAsync(b->h_off + nseg, b->tot.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+    }
     CU(cudaEventRecord(b->ev_wave[1], st));
     CU(cudaGraphLaunch(b->graph_walk, st));
+    if (tensor && (rc = launch_wave_tensor(e, T, hcap))) return rc;
     CU(cudaEventRecord(b->ev_wave[2], st));
     e->launches += WAVE_KERNELS;
     CU(cudaMemcpyAsync(e->h_pinned, b->counters.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+    if (tensor)
+      CU(cudaMemcpyAsync((uint32_t*)e->h_pinned + CNT_TENSOR, e->counters.p + CNT_TENSOR,
+                         (CNT_WORDS - CNT_TENSOR) * sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     CU(cudaStreamSynchronize(st));
+    if (tensor) {
+      bool outside = false;
+      if ((rc = tensor_status(e, &outside))) return rc;
+      if (outside) return set_err(PPS_ERR_INVALID_PARAM, "a piece outside its job's p range");
+    }
     {
       float ms0 = 0, ms1 = 0;
       CU(cudaEventElapsedTime(&ms0, b->ev_wave[0], b->ev_wave[1]));
@@ -1464,7 +1543,7 @@ extern "C" int pps_run_batch(pps_engine* e, const pps_job_params* jobs, size_t n
     bst->raw_hits = raw;
     bst->factors = nf;
     bst->waves = (uint32_t)waves;
-    bst->chunk = (uint32_t)b->tuned_work;
+    bst->chunk = (uint32_t)b->wave_work;
     bst->unroll = (uint32_t)b->walk_code & 0xffu;
     bst->primes_per_lane = (b->walk_code & WALK_TWO) ? 2u : 1u;
     float ms = 0;

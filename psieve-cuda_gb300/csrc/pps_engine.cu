@@ -234,7 +234,7 @@ extern "C" int pps_engine_create(int device, pps_engine** out) {
     e->host_seed = host_odd_primes(SEG_BITS - 1);
     if ((rc = e->seed_q.ensure(e->host_seed.size()))) break;
     if (cudaMemcpy(e->seed_q.p, e->host_seed.data(), e->host_seed.size() * 4, cudaMemcpyHostToDevice) != cudaSuccess) { rc = set_err(PPS_ERR_CUDA, "copy"); break; }
-    if ((rc = e->counters.ensure(8))) break;
+    if ((rc = e->counters.ensure(CNT_WORDS))) break;
     if ((rc = e->totals.ensure(4))) break;
   } while (0);
   if (rc) {
@@ -703,20 +703,22 @@ static int autotune(pps_engine* e, const pps_job_params* jp, const uint64_t* dP,
 // against the tensor walk's 714, N = 250,000: 861 against 740; p = 2^62, N =
 // 250,000: 711 against 761, N = 300,000: 852 against 784; p = 10^12, N =
 // 131,071: 669 against 713, N = 150,000: 764 against 724.
-static bool tensor_choice(const pps_engine* e, const pps_job_params* jp, TensorPlan* plan) {
+bool tensor_choice(const pps_engine* e, const pps_job_params* jp, TensorPlan* plan, double* saved) {
   const bool twin = jp->sign == PPS_SIGN_TWIN;
   const int v = twin ? VARIANT_TENSOR_TWIN : VARIANT_TENSOR;
   if (e->forced_variant >= 0 && e->forced_variant != v && variant_ok(jp, e->forced_variant)) return false;
   if (e->forced_split > 0 && e->forced_variant != v) return false;  // parts of the queued walks
-  if (e->forced_variant == v) return variant_ok(jp, v) && tensor_plan(jp, plan);
+  const bool forced = e->forced_variant == v;
   const double nsteps = (double)((jp->nmax - jp->nmin + jp->step - 1) / jp->step);
-  if (nsteps * 0.19 < TW_LEAST_COST) return false;  // (most short jobs, without the search for a plan)
-  return variant_ok(jp, v) && tensor_plan(jp, plan) &&
-         plan->cost < nsteps * (twin ? 0.19 : jp->step < 32 ? 0.135 : plan->digits == 4u ? 0.106 : 0.089);
+  const double old = nsteps * (twin ? 0.19 : jp->step < 32 ? 0.135 : jp->pmax <= (1ull << 47) ? 0.106 : 0.089);
+  if (!forced && old < TW_LEAST_COST) return false;  // (most short jobs, without the search for a plan)
+  if (!variant_ok(jp, v) || !tensor_plan(jp, plan)) return false;
+  if (saved) *saved = forced ? HUGE_VAL : old - plan->cost;
+  return forced || plan->cost < old;
 }
 
-static int run_tensor_walk(pps_engine* e, const pps_job_params* jp, const TensorPlan& plan, const uint64_t* dP,
-                           const uint64_t* dPinv, uint64_t np) {
+int run_tensor_walk(pps_engine* e, const pps_job_params* jp, const TensorPlan& plan, const uint64_t* dP,
+                    const uint64_t* dPinv, uint64_t np, const TensorHits& to) {
   if (int rc = e->masks.ensure(tensor_masks(plan, np))) return rc;
   TensorArgs a;
   a.P = dP;
@@ -729,16 +731,18 @@ static int run_tensor_walk(pps_engine* e, const pps_job_params* jp, const Tensor
   a.nmin = jp->nmin;
   a.nmax = jp->nmax;
   a.side = jp->sign == PPS_SIGN_TWIN ? 2u : jp->sign == 1 ? 1u : 0u;
-  a.idx_base = 0;
   a.plan = plan;
   a.batch = 0;
   a.work = e->counters.p + CNT_TENSOR;
-  a.hits = e->hits.p;
-  a.hit_count = e->counters.p;
-  a.hit_cap = hit_cap_now(e);
+  a.to = to;
   a.masks = e->masks.p;
   CU(launch_tensor_walk(a, e->num_sms, e->st, &e->launches));
   return PPS_OK;
+}
+
+// Where a one-job walk's candidates go: prime i's under idx i.
+static TensorHits job_hits(const pps_engine* e) {
+  return TensorHits{e->hits.p, e->counters.p, hit_cap_now(e), 0u, 1u};
 }
 
 // Threads per prime for the queued walk v on np primes (1 where the walk is not
@@ -809,7 +813,7 @@ extern "C" int pps_engine_set_input(pps_engine* e, const pps_input* in) {
 // The tensor walk's status words in the pinned copy of the counters: an error
 // where a bounded wait ran out; *outside is set where the caller's list held a
 // prime outside the job's range (that walk leaves it out).
-static int tensor_status(const pps_engine* e, bool* outside) {
+int tensor_status(const pps_engine* e, bool* outside) {
   const uint32_t* c = (const uint32_t*)e->h_pinned + CNT_TENSOR;
   if (c[2]) return set_err(PPS_ERR_TIMEOUT, "tensor walk: a bounded device wait expired");
   if (c[1] && outside) *outside = true;
@@ -921,7 +925,7 @@ static int run_job_once(pps_engine* e, const pps_job_params* jp, pps_factor* out
       st->split = std::max<uint32_t>(st->split, (uint32_t)split);
     }
     CU(cudaEventRecord(e->ev[2], e->st));
-    rc = tensor ? run_tensor_walk(e, jp, plan, e->P.p, e->Pinv.p, np)
+    rc = tensor ? run_tensor_walk(e, jp, plan, e->P.p, e->Pinv.p, np, job_hits(e))
                 : run_walk(e, jp, variant, e->P.p, e->Pinv.p, nullptr, np, 0, 0, (uint32_t)split);
     if (rc) return rc;
     CU(cudaEventRecord(e->ev[3], e->st));
@@ -1031,7 +1035,7 @@ static int walk_device_list(pps_engine* e, const pps_job_params* jp, const uint6
     CU(cudaMemcpyAsync(e->P.p, dP, np * sizeof(uint64_t), cudaMemcpyDefault, e->st));
     dP = e->P.p;
   }
-  const int rc = tensor ? run_tensor_walk(e, jp, plan, dP, nullptr, np)
+  const int rc = tensor ? run_tensor_walk(e, jp, plan, dP, nullptr, np, job_hits(e))
                         : run_walk(e, jp, variant, dP, nullptr, nullptr, np, 0, 0, (uint32_t)split);
   if (rc) return rc;
   CU(cudaEventRecord(e->ev[3], e->st));

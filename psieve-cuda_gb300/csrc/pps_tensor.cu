@@ -236,14 +236,14 @@ __device__ __forceinline__ void record(const TensorArgs& a, uint64_t K, uint64_t
     const uint32_t i = (uint32_t)__ffsll((long long)K) - 1u;  // K != 0
     const uint64_t k = K >> (i & 63u);
     if (i >= a.plan.s || k > a.kmax || k < a.kmin || n + i >= a.nmax) continue;
-    const uint32_t pos = atomicAdd(a.hit_count, 1u);
-    if (pos < a.hit_cap) {
+    const uint32_t pos = atomicAdd(a.to.hit_count, 1u);
+    if (pos < a.to.hit_cap) {
       pps_hit h;
       h.p = p;
       h.k = k;
       h.n = (uint32_t)n + i;
       h.idx = side ? idx | SIDE_BIT : idx;
-      a.hits[pos] = h;
+      a.to.hits[pos] = h;
     }
   }
 }
@@ -265,7 +265,7 @@ __device__ __forceinline__ void check_row(const TensorArgs& a, bool live, uint32
   const uint32_t pi = unit / a.plan.units, ta = unit - pi * a.plan.units;
   const uint32_t col = (tile - unit * ntiles) * TW_TILE + (bit >> 5) * TW_PART;
   const uint64_t p = a.P[pi], ps = a.Pinv ? a.Pinv[pi] : neg_inv64(p);
-  const uint32_t idx = a.idx_base + pi, pinv = lo32(ps);
+  const uint32_t idx = a.to.idx_base + pi * a.to.idx_step, pinv = lo32(ps);
   const uint64_t n = (uint64_t)a.nmin + (uint64_t)s * (((uint64_t)ta * TW_ROWS + row) * a.plan.nb + col);
   // its columns: of the part, of the row, of the range
   uint32_t cols = 0;
@@ -683,11 +683,11 @@ cudaError_t launch_tensor_walk(TensorArgs a, int num_sms, cudaStream_t st, uint6
   const uint64_t np = a.np, nparts = (np + part - 1) / part;
   part = nparts ? (np + nparts - 1) / nparts : 0;
   const uint64_t *P = a.P, *Pinv = a.Pinv;
-  const uint32_t idx_base = a.idx_base;
+  const uint32_t idx_base = a.to.idx_base;
   for (uint64_t at = 0; at < np; at += part) {
     a.P = P + at;
     a.Pinv = Pinv ? Pinv + at : nullptr;
-    a.idx_base = idx_base + (uint32_t)at;
+    a.to.idx_base = idx_base + (uint32_t)at * a.to.idx_step;
     a.np = std::min<uint64_t>(part, np - at);
     const uint64_t units = a.np * a.plan.units;
     // equal shares in as few batches of at most 32 units per CTA as that takes

@@ -26,6 +26,15 @@ struct TensorPlan {
 // Whether the tensor walk can run the job at all, and how.
 bool tensor_plan(const pps_job_params* jp, TensorPlan* out);
 
+// Where the candidates go, and the idx of prime i's: idx_base + i idx_step
+// (a twin candidate of the +1 side: and bit 31).
+struct TensorHits {
+  pps_hit* hits;
+  uint32_t* hit_count;
+  uint32_t hit_cap;
+  uint32_t idx_base, idx_step;
+};
+
 struct TensorArgs {
   const uint64_t* P;
   const uint64_t* Pinv;  // or null: computed
@@ -33,7 +42,6 @@ struct TensorArgs {
   uint64_t pmin, pmax, kmin, kmax;
   uint32_t nmin, nmax;
   uint32_t side;         // 1: K = -2^-n (Proth), 0: K = 2^-n (Riesel), 2: both (twin)
-  uint32_t idx_base;
   TensorPlan plan;
   uint32_t batch;        // units a CTA takes at a time (1..32)
   uint32_t* work;        // [0] batches taken (zeroed before each launch)
@@ -41,9 +49,7 @@ struct TensorArgs {
                          // [2] set when a bounded wait ran out
   uint4* masks;          // which rows pass: of each unit, tile and 32 rows a bit per row for columns 0-31,
                          // 32-63, 64-95 and 96-111 of the tile
-  pps_hit* hits;
-  uint32_t* hit_count;
-  uint32_t hit_cap;
+  TensorHits to;
 };
 
 constexpr double TW_LEAST_COST = 635.0;      // of one unit (TensorPlan::cost)
@@ -55,3 +61,11 @@ size_t tensor_masks(const TensorPlan& plan, uint64_t np);
 cudaError_t launch_tensor_walk(TensorArgs a, int num_sms, cudaStream_t st, uint64_t* launches);
 
 }  // namespace pps
+
+// (pps_engine.cu) Whether the engine takes it for the job; *saved: SM clocks per prime by the estimates.
+bool tensor_choice(const pps_engine* e, const pps_job_params* jp, pps::TensorPlan* plan, double* saved = nullptr);
+int run_tensor_walk(pps_engine* e, const pps_job_params* jp, const pps::TensorPlan& plan, const uint64_t* dP,
+                    const uint64_t* dPinv, uint64_t np, const pps::TensorHits& to);
+// The status words in the pinned copy of the counters: an error if a wait ran
+// out, *outside if a prime was outside the job's range.
+int tensor_status(const pps_engine* e, bool* outside);

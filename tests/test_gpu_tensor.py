@@ -82,3 +82,33 @@ def test_tensor_walk_in_parts(pps, engine):
         assert st.variant == variant
         got.append((st.raw_hits, fac.tobytes()))
     assert got[0] == got[1]
+
+
+@pytest.mark.parametrize("segments", [0, 4])
+def test_tensor_walk_in_a_batch(pps, segments):
+    """Long and short n ranges, one-sided and twin, in one batch: the long ones
+    leave the batch's walk kernel (with 4 segments to a wave, a part in each of
+    several waves; the first wave holds nothing else), and every job's factors
+    and counts are those of the recurrence alone."""
+    specs = [
+        dict(pmin=42 * 10**12, pmax=42 * 10**12 + 3 * 10**6, kmin=3, kmax=9999, nmin=2000, nmax=1_002_000, sign=1),
+        dict(pmin=10**12, pmax=10**12 + 10**6, kmin=3, kmax=9999, nmin=2000, nmax=5000, sign=1),
+        dict(pmin=10**12, pmax=10**12 + 2 * 10**6, kmin=3, kmax=9999, nmin=2000, nmax=602_000, sign=-1),
+        dict(pmin=42 * 10**12, pmax=42 * 10**12 + 2 * 10**6, kmin=3, kmax=9999, nmin=2000, nmax=402_000, sign=2),
+        dict(pmin=2 * 10**12, pmax=2 * 10**12 + 10**6, kmin=3, kmax=9999, nmin=3000, nmax=4000, sign=2),
+        dict(pmin=P62 - 3 * 10**6, pmax=P62 - 10**6, kmin=3, kmax=9999, nmin=100_000, nmax=900_000, sign=-1),
+    ]
+    jobs = [pps.normalize(**s) for s in specs]
+    with pps.Engine(0) as eng:
+        if segments:
+            eng.set_wave_segments(segments)
+        per, st = eng.run_batch(jobs)
+        count, total = eng.batch_job_primes(len(jobs))
+        assert st.waves >= (2 if segments else 1)
+    with pps.Engine(0) as eng:
+        for i, jp in enumerate(jobs):
+            # variant 22: twin jobs stay on the batched recurrence, alone
+            eng.set_variant(22 if specs[i]["sign"] == pps.PPS_SIGN_TWIN else 0)
+            want, one = eng.run_job(jp)
+            assert per[i].tobytes() == want.tobytes(), specs[i]
+            assert (int(count[i]), int(total[i])) == (int(one.primes), int(one.prime_sum))
