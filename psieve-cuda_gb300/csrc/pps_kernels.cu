@@ -208,30 +208,52 @@ cudaError_t launch_count_le(const uint32_t* q, uint32_t n, uint32_t x, uint32_t*
   return cudaGetLastError();
 }
 
+// The scatter's atomics are bound by the L2, and by the memory where the bitmap
+// does not fit it (129 MB on two dies): a batch of more than 3,072 segments
+// (96 MB) is scattered and sieved in equal parts.  A 2^31-wide slice (4,096
+// segments) takes 2.78 ms in two parts and took 3.14 ms in one at 4.2e13, 4.10
+// and 7.22 ms at 2^61, where the scatter has more primes.  Smaller batches
+// only pay for the second launch and its start offsets: 2,304 segments 1.63
+// against 1.58 ms (2^61: 2.59 against 2.34), 3,072 segments 2.15 against 2.09
+// (2^61: 3.22 against 3.47).
+constexpr uint32_t SIEVE_PART_SEGS = 3u << 10;
+
 int launch_sieve_batch(const SieveBatch& b, uint64_t* out64, uint64_t* pinv64, uint32_t* out32,
                        cudaStream_t st) {
   int launches = 0;
-  if (b.res && b.nq_seg > b.nq_tiny) {
-    const uint32_t n = b.nq_seg - b.nq_tiny;
-    k_sieve_res<<<(n + 255) / 256, 256, 0, st>>>(b);
+  const bool have_large = b.nq > b.nq_seg;
+  const uint32_t nparts = have_large ? (b.nseg + SIEVE_PART_SEGS - 1) / SIEVE_PART_SEGS : 1u;
+  const uint32_t segs = (b.nseg + nparts - 1) / nparts;
+  for (uint32_t s0 = 0; s0 < b.nseg; s0 += segs) {
+    SieveBatch p = b;
+    p.nseg = b.nseg - s0 < segs ? b.nseg - s0 : segs;
+    p.lo = b.lo + 2ull * s0 * SEG_BITS;
+    p.nbits = b.nbits - (uint64_t)s0 * SEG_BITS;
+    if (p.nbits > (uint64_t)p.nseg * SEG_BITS) p.nbits = (uint64_t)p.nseg * SEG_BITS;
+    p.bitmap = b.bitmap + (size_t)s0 * SEG_WORDS;
+    p.seg_count = b.seg_count + s0;
+    if (p.res && p.nq_seg > p.nq_tiny) {
+      const uint32_t n = p.nq_seg - p.nq_tiny;
+      k_sieve_res<<<(n + 255) / 256, 256, 0, st>>>(p);
+      ++launches;
+    }
+    if (have_large) {
+      cudaMemsetAsync(p.bitmap, 0xff, (size_t)p.nseg * SEG_WORDS * sizeof(uint32_t), st);
+      const uint32_t nl = p.nq - p.nq_seg;
+      uint32_t blocks = (nl + 255) / 256;
+      if (blocks > 65535u * 4u) blocks = 65535u * 4u;
+      k_sieve_large<<<blocks, 256, 0, st>>>(p);
+      ++launches;
+    }
+    k_sieve_seg<<<p.nseg, SIEVE_THREADS, 0, st>>>(p, have_large);
     ++launches;
   }
-  const int have_large = b.nq > b.nq_seg;
-  if (have_large) {
-    cudaMemsetAsync(b.bitmap, 0xff, (size_t)b.nseg * SEG_WORDS * sizeof(uint32_t), st);
-    const uint32_t nl = b.nq - b.nq_seg;
-    uint32_t blocks = (nl + 255) / 256;
-    if (blocks > 65535u * 4u) blocks = 65535u * 4u;
-    k_sieve_large<<<blocks, 256, 0, st>>>(b);
-    ++launches;
-  }
-  k_sieve_seg<<<b.nseg, SIEVE_THREADS, 0, st>>>(b, have_large);
   k_scan_counts<<<1, 1024, 0, st>>>(b.seg_count, b.seg_off, b.nseg, b.d_total);
   if (out32)
     k_expand<true><<<b.nseg, SIEVE_THREADS, 0, st>>>(b, nullptr, nullptr, out32);
   else
     k_expand<false><<<b.nseg, SIEVE_THREADS, 0, st>>>(b, out64, pinv64, nullptr);
-  launches += 3;
+  launches += 2;
   return launches;
 }
 
