@@ -45,9 +45,9 @@
 //                   pass in each 32 columns: a mask to global memory
 // and a second kernel, one thread to a passing row.
 //
-// Measured, 8.56 million primes at 4.2e13, a million n: 40.2 ms, of which the
-// second kernel 12%, against 91.0 ms of the recurrence; 6.24 million at 2^62,
-// 900,000 n: 23.5 against 47.9 ms.  What bounds the first kernel is the issue
+// Measured, 8.56 million primes at 4.2e13, a million n: 39.2 ms, of which the
+// second kernel 10%, against 91.0 ms of the recurrence; 6.24 million at 2^62,
+// 900,000 n: 23.1 against 47.9 ms.  What bounds the first kernel is the issue
 // of instructions (3,460 a prime, 71% of the slots, the integer pipe 73% busy),
 // no longer multiplies: about 90 a warp and test tile, of them 32 the minima,
 // 50 a B row warp, 200 an A warp.  Its chains come close behind: the build warps
@@ -256,10 +256,27 @@ __device__ __forceinline__ uint64_t halve(uint64_t K, uint32_t s, uint32_t low, 
   return mk64(__funnelshift_rc(lo32(u), lo32(v), s), __funnelshift_rc(lo32(v), hi32(v), s));
 }
 
+// 2^-e mod p, e >= 32, odd p < 2^62, pi = p^-1 mod 2^64: inv_pow2 (pps_device.cuh)
+// with the residues below 2p, so that a product needs no comparison: hi < p and
+// m p's high word < p give hi - high + p in (0, 2p).  With it, and a kernel for
+// each kind of scan, the second kernel took 147 clocks a prime instead of 190 in
+// the first case above (380 warp instructions a prime instead of 442).
+__device__ __forceinline__ uint64_t inv_pow2_wide(uint32_t e, uint64_t p, uint64_t pi) {
+  int b = 26 - __clz(e);
+  uint64_t r = 1ull << (64 - (e >> b));
+  for (--b; b >= 0; --b) {
+    r = __umul64hi(r, r) - __umul64hi(r * r * pi, p) + p;
+    if ((e >> b) & 1u) r = (r + (r & 1ull ? p : 0ull)) >> 1;
+  }
+  return p - __umul64hi(r * pi, p);
+}
+
 // Row `bit` of word `at` of the masks: K at the first of its columns, then
 // column by column, exactly.  Whole warps (live: whether the lane has a row).
+// TWIN: both sides; LONG: s above 32, in two steps.
+template <bool TWIN, bool LONG>
 __device__ __forceinline__ void check_row(const TensorArgs& a, bool live, uint32_t at, uint32_t bit, uint32_t ntiles) {
-  const uint32_t s = a.plan.s, s2 = s > 32u ? s - 32u : s, low = 0xffffffffu >> (32u - s2);
+  const uint32_t s = a.plan.s, s2 = LONG ? s - 32u : s, low = 0xffffffffu >> (32u - s2);
   const uint64_t most = (uint64_t)a.kmax << (s - 1u);  // of a K that can be a hit (tensor_plan: below p)
   const uint32_t tile = at >> 2, unit = tile / ntiles, row = (at & 3u) * 32u + (bit & 31u);
   const uint32_t pi = unit / a.plan.units, ta = unit - pi * a.plan.units;
@@ -271,8 +288,8 @@ __device__ __forceinline__ void check_row(const TensorArgs& a, bool live, uint32
   uint32_t cols = 0;
   if (live && n < a.nmax)
     cols = min(min(bit < 96u ? TW_PART : TW_TILE - 3u * TW_PART, a.plan.nb - col), (uint32_t)((a.nmax - 1u - n) / s) + 1u);
-  uint64_t K = inv_pow2((uint32_t)n, p, ps);
-  if (a.side == 1u) K = p - K;
+  uint64_t K = inv_pow2_wide((uint32_t)n, p, 0ull - ps);
+  if (!TWIN && a.side == 1u) K = p - K;
   const uint64_t K0 = K;
   const uint32_t all = __reduce_max_sync(0xffffffffu, cols);
   // the last K that is small enough, and how many are
@@ -280,26 +297,27 @@ __device__ __forceinline__ void check_row(const TensorArgs& a, bool live, uint32
   uint32_t found_b = 0, count = 0;
 #pragma unroll 2
   for (uint32_t b = 0; b < all; ++b) {
-    if ((K <= most || (a.side == 2u && p - K <= most)) && b < cols) {
+    if ((K <= most || (TWIN && p - K <= most)) && b < cols) {
       found = K;
       found_b = b;
       ++count;
     }
-    if (s > 32u) K = halve(K, 32u, 0xffffffffu, p, pinv);
+    if (LONG) K = halve(K, 32u, 0xffffffffu, p, pinv);
     K = halve(K, s2, low, p, pinv);
   }
   if (count) record(a, found, n + (uint64_t)s * found_b, p, idx);
   if (count > 1u) {
     K = K0;
     for (uint32_t b = 0; b < found_b; ++b) {
-      if (K <= most || (a.side == 2u && p - K <= most)) record(a, K, n + (uint64_t)s * b, p, idx);
-      if (s > 32u) K = halve(K, 32u, 0xffffffffu, p, pinv);
+      if (K <= most || (TWIN && p - K <= most)) record(a, K, n + (uint64_t)s * b, p, idx);
+      if (LONG) K = halve(K, 32u, 0xffffffffu, p, pinv);
       K = halve(K, s2, low, p, pinv);
     }
   }
 }
 
 // The rows that pass, of masks[0, n): a warp collects 32 and takes one in each lane.
+template <bool TWIN, bool LONG>
 __global__ void __launch_bounds__(256) k_tensor_check(const __grid_constant__ TensorArgs a, uint32_t n, uint32_t ntiles) {
   __shared__ uint32_t queue[8][64];
   uint32_t* const q = queue[threadIdx.x >> 5];
@@ -321,14 +339,14 @@ __global__ void __launch_bounds__(256) k_tensor_check(const __grid_constant__ Te
         if (have < 32u) continue;
         have -= 32u;
         const uint32_t e = q[lane];
-        check_row(a, true, e >> 7, e & 127u, ntiles);
+        check_row<TWIN, LONG>(a, true, e >> 7, e & 127u, ntiles);
         __syncwarp();
         if (lane < have) q[lane] = q[32u + lane];
         __syncwarp();
       }
     }
   }
-  if (have) check_row(a, lane < have, q[lane < have ? lane : 0u] >> 7, q[lane < have ? lane : 0u] & 127u, ntiles);
+  if (have) check_row<TWIN, LONG>(a, lane < have, q[lane < have ? lane : 0u] >> 7, q[lane < have ? lane : 0u] & 127u, ntiles);
 }
 
 // Both 16-bit minima of 8 and of 16 registers.
@@ -675,6 +693,9 @@ size_t tensor_masks(const TensorPlan& plan, uint64_t np) {
 
 cudaError_t launch_tensor_walk(TensorArgs a, int num_sms, cudaStream_t st, uint64_t* launches) {
   auto fn = a.plan.digits == 4u ? k_tensor_walk<4> : k_tensor_walk<5>;
+  const bool twin = a.side == 2u, lng = a.plan.s > 32u;
+  auto check = twin ? (lng ? k_tensor_check<true, true> : k_tensor_check<true, false>)
+                    : (lng ? k_tensor_check<false, true> : k_tensor_check<false, false>);
   const size_t smem = tensor_smem(a.plan.nb, a.plan.pitch);
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
@@ -699,7 +720,7 @@ cudaError_t launch_tensor_walk(TensorArgs a, int num_sms, cudaStream_t st, uint6
     if ((e = cudaMemsetAsync(a.work, 0, sizeof(uint32_t), st)) != cudaSuccess) return e;
     fn<<<grid, TW_THREADS, smem, st>>>(a);
     const uint32_t masks = (uint32_t)units * ntiles * 4u;
-    k_tensor_check<<<(int)std::min<uint32_t>((masks + 255u) / 256u, 8u * (uint32_t)num_sms), 256, 0, st>>>(a, masks, ntiles);
+    check<<<(int)std::min<uint32_t>((masks + 255u) / 256u, 8u * (uint32_t)num_sms), 256, 0, st>>>(a, masks, ntiles);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     *launches += 2;
   }
