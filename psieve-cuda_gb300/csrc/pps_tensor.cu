@@ -45,12 +45,12 @@
 //                   pass in each 32 columns: a mask to global memory
 // and a second kernel, one thread to a passing row.
 //
-// Measured, 8.56 million primes at 4.2e13, a million n: 39.2 ms, of which the
+// Measured, 8.56 million primes at 4.2e13, a million n: 38.7 ms, of which the
 // second kernel 10%, against 91.0 ms of the recurrence; 6.24 million at 2^62,
-// 900,000 n: 23.1 against 47.9 ms.  What bounds the first kernel is the issue
+// 900,000 n: 22.3 against 47.9 ms.  What bounds the first kernel is the issue
 // of instructions (3,460 a prime, 71% of the slots, the integer pipe 73% busy),
 // no longer multiplies: about 90 a warp and test tile, of them 32 the minima,
-// 50 a B row warp, 200 an A warp.  Its chains come close behind: the build warps
+// 45 a B row warp, 190 an A warp.  Its chains come close behind: the build warps
 // spend 60% of a prime's 1,300 clocks on their rows (a third group took the
 // cases above from 41.7 and 26.7 ms), a test warp 70% on its tile.  The MMAs
 // fill 224 clocks.  A tile in one load, which frees it sooner but holds 24
@@ -188,12 +188,10 @@ __device__ __forceinline__ uint32_t digits_up(uint32_t v, uint32_t mask, uint32_
   return *reinterpret_cast<const uint32_t*>(&d);
 }
 
-// B's row of column b: the balanced digits of v_b from the expansion's words
-// at bit s b, slots in the order of a_row.
+// B's row of column b: the balanced digits of v_b from the expansion's bits from
+// s b on, bit sh of w[0], slots in the order of a_row.
 template <int G>
-__device__ __forceinline__ void b_row(const uint32_t* S, uint32_t bit, uint32_t* r) {
-  const uint32_t* w = S + (bit >> 5);
-  const uint32_t sh = bit & 31u;
+__device__ __forceinline__ void b_row(const uint32_t* w, uint32_t sh, uint32_t* r) {
   if (G == 4) {
     uint32_t q0 = __funnelshift_r(w[0], w[1], sh), q1 = __funnelshift_r(w[1], w[2], sh);
     asm("add.cc.u32 %0, %0, 0x88888888;\n\taddc.u32 %1, %1, 0x88888888;" : "+r"(q0), "+r"(q1));
@@ -455,6 +453,7 @@ __global__ void __launch_bounds__(TW_THREADS, 1) k_tensor_walk(const __grid_cons
   } else if (warp < TW_TEST_WARPS + TW_BUILD_WARPS) {
     // ------------------------------------------------------------ build
     const uint32_t group = (warp - TW_TEST_WARPS) >> 2, quarter = (warp & 3u) * 32u, row = quarter + lane;
+    const uint32_t bit = (s * row) & 31u;
     uint32_t unit_no = 0;
     bool ok = true;
     for (uint32_t it = 0; ok; ++it) {
@@ -470,11 +469,13 @@ __global__ void __launch_bounds__(TW_THREADS, 1) k_tensor_walk(const __grid_cons
         const uint32_t* Sp = S + ((size_t)slot * 32u + unit) * pitch;
         uint4* b4 = reinterpret_cast<uint4*>(bop) + st * 2u * nbp;
         // two B rows at a time where there are: independent work to fill each other's latencies
+        // (128 rows on are 4 s words on, at the same bit)
+        const uint32_t* w = Sp + ((s * row) >> 5);
         uint32_t b = row;
-        for (; b + TW_ROWS < nb; b += 2u * TW_ROWS) {
+        for (; b + TW_ROWS < nb; b += 2u * TW_ROWS, w += 8u * s) {
           uint32_t r[8], r2[8];
-          b_row<G>(Sp, s * b, r);
-          b_row<G>(Sp, s * (b + TW_ROWS), r2);
+          b_row<G>(w, bit, r);
+          b_row<G>(w + 4u * s, bit, r2);
           b4[b] = make_uint4(r[0], r[1], r[2], r[3]);
           b4[nbp + b] = make_uint4(r[4], r[5], r[6], r[7]);
           b4[b + TW_ROWS] = make_uint4(r2[0], r2[1], r2[2], r2[3]);
@@ -482,16 +483,21 @@ __global__ void __launch_bounds__(TW_THREADS, 1) k_tensor_walk(const __grid_cons
         }
         if (b < nb) {
           uint32_t r[8];
-          b_row<G>(Sp, s * b, r);
+          b_row<G>(w, bit, r);
           b4[b] = make_uint4(r[0], r[1], r[2], r[3]);
           b4[nbp + b] = make_uint4(r[4], r[5], r[6], r[7]);
         }
         {
           uint32_t r[16];
           const uint64_t p = tab[TAB_P];
-          uint64_t K = mont_mul(tab[row >> 4], tab[TAB_H + (row & 15u)], p, tab[TAB_PS]);
-          if (K > p >> 1) K -= p;  // the nearer one to 0 (mod 2^64): half of v_b's error
-          a_row<G>(K, a.plan.off, r);
+          // the product in (-p, p), no comparison (as inv_pow2_wide), then the residue
+          // nearest to 0: half of v_b's error
+          const uint64_t g = tab[row >> 4], h = tab[TAB_H + (row & 15u)];
+          int64_t K = (int64_t)(__umul64hi(g, h) - __umul64hi(g * h * (0ull - tab[TAB_PS]), p));
+          const int64_t hp = (int64_t)(p >> 1);
+          if (K > hp) K -= (int64_t)p;
+          if (K < -hp) K += (int64_t)p;
+          a_row<G>((uint64_t)K, a.plan.off, r);
           tc_fence_after();
           tmem_st16(tmem + (quarter << 16) + TW_ACOL + st * 16u, r);
         }
