@@ -41,6 +41,7 @@ constexpr uint32_t WAVE_BATCHES = WAVE_SEGS;    // at most one batch per segment
 constexpr uint32_t MAX_JOBS = 1u << 16;
 constexpr int BW_THREADS = 256;
 constexpr uint32_t BQ_CAP = 512;  // queued blocks per warp
+constexpr uint32_t WAVE_WARPS = 32;   // work items that keep an SM busy, one to a warp
 constexpr uint32_t MAX_CHUNK = 8192;  // primes per work chunk, at most (a multiple of 32)
 
 struct BJob {
@@ -1356,6 +1357,16 @@ int batch_wave(pps_engine* e, const BatchPiece* pieces, size_t n, std::vector<pp
   // (a first wave of the tensor walk's jobs alone has timed nothing)
   b->walk_code = e->forced_bwalk ? e->forced_bwalk : b->tuned_unroll ? b->tuned_unroll : 8 | WALK_TWO;
   b->wave_work = b->tuned_work ? b->tuned_work : 1024;
+  // Smaller chunks where the wave would leave warps idle: the choice may have been
+  // timed on a wave of other jobs, and a short job of a few chunks runs at the
+  // speed of one warp (a twin job of 2,660 primes and 4,849 n: 272 us in chunks of
+  // 256 steps, 304 us in chunks of 1,024).
+  double steps = 0;
+  for (uint32_t i = 0; i < nb; ++i) {
+    const BJob& J = b->hjobs[T->batch[i].job];
+    if (!J.tensor) steps += 2.0 * (double)T->batch[i].nbits / log((double)T->batch[i].lo) * J.nsteps;
+  }
+  while (b->wave_work > 256 && steps < 32.0 * b->wave_work * WAVE_WARPS * e->num_sms) b->wave_work /= 4;
   if ((rc = set_chunks(e, smin, smax, b->wave_work))) return rc;
 
   // the wave itself: a captured graph of the fixed sequence, replayed

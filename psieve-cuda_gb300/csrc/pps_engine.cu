@@ -825,7 +825,7 @@ int tensor_status(const pps_engine* e, bool* outside) {
 // buffer), so the two counts come back in one copy after it: a raw count
 // beyond the buffer then means an overflow (the call walks again).
 static int finish_job(pps_engine* e, const pps_job_params* jp, pps_factor* out, size_t cap, size_t* nout,
-                      pps_job_stats* st, uint32_t* raw_hits_out, bool* overflow, bool* outside = nullptr) {
+                      pps_job_stats* st, uint32_t* raw_hits_out, bool* overflow, bool tensor, bool* outside = nullptr) {
   if (int rc = ensure_input_keys(e, jp)) return rc;
   FilterArgs f;
   f.hits = e->hits.p;
@@ -854,10 +854,13 @@ static int finish_job(pps_engine* e, const pps_job_params* jp, pps_factor* out, 
   CU(launch_filter(f, (uint32_t)e->num_sms * 8u, e->st));
   e->launches++;
   CU(cudaEventRecord(e->ev[5], e->st));
-  CU(cudaMemcpyAsync(e->h_pinned, e->counters.p, CNT_WORDS * sizeof(uint32_t), cudaMemcpyDeviceToHost, e->st));
+  CU(cudaMemcpyAsync(e->h_pinned, e->counters.p, (tensor ? CNT_WORDS : 2u) * sizeof(uint32_t), cudaMemcpyDeviceToHost,
+                     e->st));
   CU(cudaStreamSynchronize(e->st));
-  if (int rc = tensor_status(e, outside)) return rc;
-  if (outside && *outside) return PPS_OK;  // the caller walks its list again
+  if (tensor) {
+    if (int rc = tensor_status(e, outside)) return rc;
+    if (outside && *outside) return PPS_OK;  // the caller walks its list again
+  }
   const uint32_t raw = ((uint32_t*)e->h_pinned)[0];
   *raw_hits_out = raw;
   if (raw > hit_cap_now(e)) {
@@ -889,10 +892,10 @@ static int run_job_once(pps_engine* e, const pps_job_params* jp, pps_factor* out
   BaseTable bt;
   int rc = prepare_sieving_primes(e, jp->qmax, jp->pmax, &dq, &bt);
   if (rc) return rc;
-  CU(cudaMemsetAsync(e->counters.p, 0, CNT_WORDS * sizeof(uint32_t), e->st));
   int variant = -1;
   TensorPlan plan;
   const bool tensor = tensor_choice(e, jp, &plan);
+  CU(cudaMemsetAsync(e->counters.p, 0, (tensor ? CNT_WORDS : 2u) * sizeof(uint32_t), e->st));
   if (tensor) variant = jp->sign == PPS_SIGN_TWIN ? VARIANT_TENSOR_TWIN : VARIANT_TENSOR;
   const uint64_t span = e->batch_span;
   for (uint64_t a = jp->pmin | 1ull; a < jp->pmax; a += span) {
@@ -941,7 +944,7 @@ static int run_job_once(pps_engine* e, const pps_job_params* jp, pps_factor* out
     }
   }
   uint32_t raw = 0;
-  rc = finish_job(e, jp, out, cap, nout, st, &raw, overflow);
+  rc = finish_job(e, jp, out, cap, nout, st, &raw, overflow, tensor);
   if (st) st->raw_hits = raw;
   return rc;
 }
@@ -1017,9 +1020,10 @@ extern "C" int pps_run_job(pps_engine* e, const pps_job_params* jp, pps_factor* 
 // primes lie in [pmin, pmax), or the tensor walk, which needs that, has not
 // found otherwise yet.
 static int walk_device_list(pps_engine* e, const pps_job_params* jp, const uint64_t* dP, size_t np,
-                            pps_job_stats* st, bool in_range) {
+                            pps_job_stats* st, bool in_range, bool* is_tensor) {
   TensorPlan plan;
   const bool tensor = in_range && tensor_choice(e, jp, &plan);
+  *is_tensor = tensor;
   const int variant = !tensor ? autotune(e, jp, dP, nullptr, np)
                               : jp->sign == PPS_SIGN_TWIN ? VARIANT_TENSOR_TWIN : VARIANT_TENSOR;
   if (variant < 0) return variant;
@@ -1028,6 +1032,8 @@ static int walk_device_list(pps_engine* e, const pps_job_params* jp, const uint6
   if (split < 0) return split;
   if (st) st->split = (uint32_t)split;
   CU(cudaEventRecord(e->ev[2], e->st));
+  if (tensor)
+    CU(cudaMemsetAsync(e->counters.p + CNT_TENSOR, 0, (CNT_WORDS - CNT_TENSOR) * sizeof(uint32_t), e->st));
   cudaPointerAttributes at;
   if (tensor && cudaPointerGetAttributes(&at, dP) == cudaSuccess && at.type == cudaMemoryTypeHost) {
     // a page-locked list: its re-check would read some primes a few times more
@@ -1063,11 +1069,11 @@ extern "C" int pps_check_primes_device(pps_engine* e, const pps_job_params* jp, 
     if (rc) return rc;
     e->hit_cap_limit = attempt == 0 ? debug_first_hit_cap() : 0;
     if (st) memset(st, 0, sizeof *st);
-    CU(cudaMemsetAsync(e->counters.p, 0, CNT_WORDS * sizeof(uint32_t), e->st));
-    if (np && (rc = walk_device_list(e, jp, d_P, np, st, in_range))) return rc;
-    bool overflow = false, outside = false;
+    CU(cudaMemsetAsync(e->counters.p, 0, 2 * sizeof(uint32_t), e->st));
+    bool tensor = false, overflow = false, outside = false;
+    if (np && (rc = walk_device_list(e, jp, d_P, np, st, in_range, &tensor))) return rc;
     uint32_t raw = 0;
-    rc = finish_job(e, jp, out, cap, nout, st, &raw, &overflow, &outside);
+    rc = finish_job(e, jp, out, cap, nout, st, &raw, &overflow, tensor, &outside);
     if (st) st->raw_hits = raw;
     if (!rc && outside) {  // not an attempt: the list is walked by the recurrence from here on
       in_range = false;
@@ -1085,7 +1091,7 @@ extern "C" int pps_check_primes_device(pps_engine* e, const pps_job_params* jp, 
 }
 
 // The device address of a caller's host list of primes.  A page-locked
-// (pinned) buffer is read in place by the walk over the host link: each prime
+// (pinned) buffer is read in place by the recurrence over the host link: each prime
 // is loaded once, 8 B per prime, a small fraction of the link's bandwidth at
 // the walk's rate.  Any other host buffer is first copied into the engine's
 // device list.
@@ -1134,12 +1140,13 @@ extern "C" int pps_check_primes_raw(pps_engine* e, const pps_job_params* jp, con
   for (int attempt = 0; attempt < 4; ++attempt) {
     if ((rc = ensure_hit_buffers(e, hit_cap, std::max<size_t>(1u << 18, e->factors.n)))) return rc;
     e->hit_cap_limit = attempt == 0 ? debug_first_hit_cap() : 0;
-    CU(cudaMemsetAsync(e->counters.p, 0, CNT_WORDS * sizeof(uint32_t), e->st));
-    if (np && (rc = walk_device_list(e, jp, dP, np, nullptr, in_range))) return rc;
-    CU(cudaMemcpyAsync(e->h_pinned, e->counters.p, CNT_WORDS * sizeof(uint32_t), cudaMemcpyDeviceToHost, e->st));
+    CU(cudaMemsetAsync(e->counters.p, 0, 2 * sizeof(uint32_t), e->st));
+    bool tensor = false, outside = false;
+    if (np && (rc = walk_device_list(e, jp, dP, np, nullptr, in_range, &tensor))) return rc;
+    CU(cudaMemcpyAsync(e->h_pinned, e->counters.p, (tensor ? CNT_WORDS : 1u) * sizeof(uint32_t),
+                       cudaMemcpyDeviceToHost, e->st));
     CU(cudaStreamSynchronize(e->st));
-    bool outside = false;
-    if ((rc = tensor_status(e, &outside))) return rc;
+    if (tensor && (rc = tensor_status(e, &outside))) return rc;
     if (outside) {  // not an attempt: the list is walked by the recurrence from here on
       in_range = false;
       --attempt;
