@@ -14,14 +14,18 @@ larger than the 129 MB L2, so no flush is needed between steps).
 value  = primes fully walked per second (whole job, all ranks).
 e2e    = the same metric through the drop-in C-ABI call with HOST buffers:
          pps_check_primes() given the slice's primes in pinned host memory
-         (read by the walk in place over the host link, inside the timed
-         region) and returning the factor list to the host (D2H inside the
-         timed region) -- what the reference's check_ns / get_factors_found
-         boundary carries.
-roofline: the walk kernel is bound by the 32-bit integer multiply pipe; its
-         algorithmic work is 3 multiplies per walk step (one 32 n-values advance
-         of one prime); the peak is the multiply-pipe throughput measured in this
-         run by pps_measure_imad_peak on the same multiply mix.
+         (copied to the device by the tensor walk's call, read in place over
+         the host link by the recurrence, inside the timed region) and
+         returning the factor list to the host (D2H inside the timed region) --
+         what the reference's check_ns / get_factors_found boundary carries.
+roofline: the tensor walk is bound by the issue of instructions; its work is the
+         warp instructions per prime of its committed profile, the peak four a
+         clock and SM at the clock sampled in this run; beside it the rate of its
+         matrix products.  The recurrence is bound by the 32-bit integer
+         multiply pipe; its algorithmic work is 3 multiplies per walk step (one
+         32 n-values advance of one prime); the peak is the multiply-pipe
+         throughput measured in this run by pps_measure_imad_peak on the same
+         multiply mix.
 verify : the checker leg, after every timed leg and not timed: the large-n
          Proth workload (47 slices) and the 62-bit Riesel workload
          (p in [2^62 - 2^34, 2^62), 8 slices) run in full on the GPU; every
@@ -149,14 +153,14 @@ class Clocks:
                 "samples": len(sm)}
 
 
-def _traffic_from_profile(kernel: str) -> float | None:
-    """DRAM bytes per prime of the walk kernel from the committed ncu summary of
-    that kernel (the walk reads each prime's 16 B once, whatever the n range)."""
+def _from_profile(kernel: str, key: str = "dram_bytes_per_prime") -> float | None:
+    """A figure per prime of the walk kernel from the committed ncu summary of
+    that kernel on the large-n range: its DRAM bytes, warp instructions or flop."""
     f = ROOT / "profiles" / f"{kernel}_large_n.md"
     if not f.exists():
         return None
     for line in f.read_text().splitlines():
-        if line.startswith("dram_bytes_per_prime:"):
+        if line.startswith(key + ":"):
             return float(line.split(":")[1])
     return None
 
@@ -872,23 +876,34 @@ def run_gpu(args) -> None:
         return
 
     # ---- roofline of the walk kernel
-    peak_mults = eng.imad_peak()
-    mults = 3.0 * steps_done
-    achieved = mults / (walk_ms * 1e-3)
     variant = stats[-1].variant if stats else 0
     kernel = ppsgpu.walk_kernel_name(variant)
-    traffic = _traffic_from_profile(kernel)
+    traffic = _from_profile(kernel)
     peaks = _measured_peaks()
+    tensor = None
+    if kernel == "k_tensor_walk":
+        instr, flop = _from_profile(kernel, "warp_instructions_per_prime"), _from_profile(kernel, "mma_flop_per_prime")
+        mhz = clk.summary()["sm_mhz"] or peaks.get("sm_max_mhz") or 0.0
+        bound, unit, per = "issue", "G warp instructions/s", f"{instr} warp instructions per prime (ncu)"
+        achieved, peak = (instr or 0.0) * primes / (walk_ms * 1e-3), 4.0 * mhz * 1e6 * torch.cuda.get_device_properties(local).multi_processor_count
+        source = "4 a clock and SM at the median SM clock of this run"
+        rate, tf = (flop or 0.0) * primes / (walk_ms * 1e-3) / 1e12, peaks.get("bf16_tflops")
+        tensor = {"bound": "tensor", "achieved": rate, "peak": tf, "unit": "TFLOP/s", "frac": rate / tf if tf else None,
+                  "peak_source": "MEASURED_PEAKS.json bf16_tflops (of measured)",
+                  "work_per_unit": f"{flop} flop of fp16 matrix products per prime"}
+    else:
+        bound, unit, per = "imad", "Gmul/s", "3 multiplies per walk step (one prime advanced by 32 n)"
+        achieved, peak = 3.0 * steps_done / (walk_ms * 1e-3), eng.imad_peak()
+        source = "measured in this run (pps_measure_imad_peak)"
     hbm = peaks.get("hbm_gbs")
     sieve_gbs = 16.0 * primes / (sieve_ms * 1e-3) / 1e9 if sieve_ms > 0 else None
-    launches_walk = len(stats)  # one walk launch per job
-    roofline = {"bound": "imad", "achieved": achieved / 1e9, "peak": peak_mults / 1e9,
-                "unit": "Gmul/s", "frac": achieved / peak_mults,
-                "traffic": (traffic * primes / launches_walk) if traffic else None,
-                "traffic_unit": "bytes per launch (ncu DRAM bytes per prime x primes per launch)",
+    walks = len(stats)  # one walk per job (the tensor walk in several launches)
+    roofline = {"bound": bound, "achieved": achieved / 1e9, "peak": peak / 1e9,
+                "unit": unit, "frac": achieved / peak if peak else None,
+                "traffic": (traffic * primes / walks) if traffic else None,
+                "traffic_unit": "bytes per walk of a slice (ncu DRAM bytes per prime x its primes)",
                 "kernel": f"{kernel} (variant {variant}: {ppsgpu.walk_variant_name(variant)})",
-                "peak_source": "measured in this run (pps_measure_imad_peak)",
-                "work_per_unit": "3 multiplies per walk step (one prime advanced by 32 n)",
+                "peak_source": source, "work_per_unit": per, "tensor": tensor,
                 "sieve": {"bound": "hbm", "achieved": sieve_gbs, "peak": hbm, "unit": "GB/s",
                           "frac": (sieve_gbs / hbm) if (sieve_gbs and hbm) else None,
                           "peak_source": "MEASURED_PEAKS.json hbm_gbs (of measured)",
