@@ -1178,7 +1178,7 @@ int batch_set_jobs(pps_engine* e, uint32_t slot0, const pps_job_params* jobs, si
     TensorSlot t;
     double saved = 0;
     b->tensor.erase((uint32_t)(slot0 + j));
-    if (!e->forced_bwalk && tensor_choice(e, &jobs[j], &t.plan, &saved) &&
+    if (!e->forced_bwalk && tensor_choice(e, &jobs[j], 0, &t.plan, &saved) &&
         saved * (double)(jobs[j].pmax - jobs[j].pmin) > TENSOR_LEAST_SAVED * log((double)jobs[j].pmin)) {
       t.job = jobs[j];
       J.tensor = 1;

@@ -703,7 +703,15 @@ static int autotune(pps_engine* e, const pps_job_params* jp, const uint64_t* dP,
 // against the tensor walk's 714, N = 250,000: 861 against 740; p = 2^62, N =
 // 250,000: 711 against 761, N = 300,000: 852 against 784; p = 10^12, N =
 // 131,071: 669 against 713, N = 150,000: 764 against 724.
-bool tensor_choice(const pps_engine* e, const pps_job_params* jp, TensorPlan* plan, double* saved) {
+// With few primes (np > 0) the calls' times decide: the tensor walk's launches,
+// first seeds and tail are about 55,000 clocks (27 us), its share of the call's
+// host time 5 us more; the recurrence takes a fifth longer on less than a third
+// of its resident threads, and cannot be faster than one thread's eighth of the
+// n range, 58 clocks a step (38 for the shorter steps).  Over 252 calls of 300
+// to 400,000 primes and 100,000 to 700,000 n this takes the slower walk nowhere
+// by more than the calls' own spread; by the estimates above alone 3,000 primes
+// at 10^12, 150,000 n took 27 us instead of 22.
+bool tensor_choice(const pps_engine* e, const pps_job_params* jp, double np, TensorPlan* plan, double* saved) {
   const bool twin = jp->sign == PPS_SIGN_TWIN;
   const int v = twin ? VARIANT_TENSOR_TWIN : VARIANT_TENSOR;
   if (e->forced_variant >= 0 && e->forced_variant != v && variant_ok(jp, e->forced_variant)) return false;
@@ -714,7 +722,16 @@ bool tensor_choice(const pps_engine* e, const pps_job_params* jp, TensorPlan* pl
   if (!forced && old < TW_LEAST_COST) return false;  // (most short jobs, without the search for a plan)
   if (!variant_ok(jp, v) || !tensor_plan(jp, plan)) return false;
   if (saved) *saved = forced ? HUGE_VAL : old - plan->cost;
-  return forced || plan->cost < old;
+  if (forced || np <= 0) return forced || plan->cost < old;
+  const double primes = np / e->num_sms;  // of one SM
+  return primes * plan->cost + 66000.0 < std::max(primes * old * (np < 64000.0 ? 1.2 : 1.0),
+                                                  nsteps / 8.0 * (jp->step < 32 ? 38.0 : 58.0) + 20000.0);
+}
+
+// About how many primes a batch of the job's range holds.
+static double job_primes(const pps_engine* e, const pps_job_params* jp) {
+  if (jp->pmax <= jp->pmin) return 0;
+  return (double)std::min(jp->pmax - jp->pmin, e->batch_span) / log((double)jp->pmin);
 }
 
 int run_tensor_walk(pps_engine* e, const pps_job_params* jp, const TensorPlan& plan, const uint64_t* dP,
@@ -894,7 +911,7 @@ static int run_job_once(pps_engine* e, const pps_job_params* jp, pps_factor* out
   if (rc) return rc;
   int variant = -1;
   TensorPlan plan;
-  const bool tensor = tensor_choice(e, jp, &plan);
+  const bool tensor = tensor_choice(e, jp, job_primes(e, jp), &plan);
   CU(cudaMemsetAsync(e->counters.p, 0, (tensor ? CNT_WORDS : 2u) * sizeof(uint32_t), e->st));
   if (tensor) variant = jp->sign == PPS_SIGN_TWIN ? VARIANT_TENSOR_TWIN : VARIANT_TENSOR;
   const uint64_t span = e->batch_span;
@@ -982,7 +999,7 @@ extern "C" int pps_run_job(pps_engine* e, const pps_job_params* jp, pps_factor* 
     // except with an input file: its rule applies on the one-job path, whose
     // twin kernels need 32-bit steps or p <= 2^(32+s)
     TensorPlan plan;
-    if (!e->input && !tensor_choice(e, jp, &plan)) return run_twin_job(e, jp, out, cap, nout, st);
+    if (!e->input && !tensor_choice(e, jp, job_primes(e, jp), &plan)) return run_twin_job(e, jp, out, cap, nout, st);
     bool exact = false;
     for (int v = 0; v < PPS_NUM_VARIANTS && !exact; ++v) exact = variant_ok(jp, v) != 0;
     if (!exact)
@@ -1022,7 +1039,7 @@ extern "C" int pps_run_job(pps_engine* e, const pps_job_params* jp, pps_factor* 
 static int walk_device_list(pps_engine* e, const pps_job_params* jp, const uint64_t* dP, size_t np,
                             pps_job_stats* st, bool in_range, bool* is_tensor) {
   TensorPlan plan;
-  const bool tensor = in_range && tensor_choice(e, jp, &plan);
+  const bool tensor = in_range && tensor_choice(e, jp, (double)np, &plan);
   *is_tensor = tensor;
   const int variant = !tensor ? autotune(e, jp, dP, nullptr, np)
                               : jp->sign == PPS_SIGN_TWIN ? VARIANT_TENSOR_TWIN : VARIANT_TENSOR;

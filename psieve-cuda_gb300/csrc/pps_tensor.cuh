@@ -62,8 +62,10 @@ cudaError_t launch_tensor_walk(TensorArgs a, int num_sms, cudaStream_t st, uint6
 
 }  // namespace pps
 
-// (pps_engine.cu) Whether the engine takes it for the job; *saved: SM clocks per prime by the estimates.
-bool tensor_choice(const pps_engine* e, const pps_job_params* jp, pps::TensorPlan* plan, double* saved = nullptr);
+// (pps_engine.cu) Whether the engine takes it for np primes of the job (0: as many as fill the GPU); *saved:
+// SM clocks per prime by the estimates.
+bool tensor_choice(const pps_engine* e, const pps_job_params* jp, double np, pps::TensorPlan* plan,
+                   double* saved = nullptr);
 int run_tensor_walk(pps_engine* e, const pps_job_params* jp, const pps::TensorPlan& plan, const uint64_t* dP,
                     const uint64_t* dPinv, uint64_t np, const pps::TensorHits& to);
 // The status words in the pinned copy of the counters: an error if a wait ran
