@@ -91,7 +91,7 @@ constexpr uint32_t TAB_H = 8, TAB_P = 24, TAB_PS = 25, TAB_PITCH = 27;  // words
 constexpr uint32_t SIDE_BIT = 0x80000000u;  // a twin candidate of the +1 side
 
 struct __align__(128) Shared {
-  uint64_t seed_full[2], seed_empty[2];
+  uint64_t seed_full[2], seed_empty[2], taken[2];
   uint64_t ab_full[TW_STAGES], ab_empty[TW_STAGES];
   uint64_t d_full[TW_GROUPS], d_empty[TW_GROUPS / 2];
   uint64_t first[2];
@@ -377,6 +377,7 @@ __global__ void __launch_bounds__(TW_THREADS, 1) k_tensor_walk(const __grid_cons
     for (int i = 0; i < 2; ++i) {
       mbar_init(smem_addr(&sh->seed_full[i]), TW_SEED_WARPS);
       mbar_init(smem_addr(&sh->seed_empty[i]), TW_THREADS / 32 - TW_SEED_WARPS);
+      mbar_init(smem_addr(&sh->taken[i]), 1);
     }
     for (uint32_t i = 0; i < TW_STAGES; ++i) {
       mbar_init(smem_addr(&sh->ab_full[i]), 4);
@@ -526,13 +527,22 @@ __global__ void __launch_bounds__(TW_THREADS, 1) k_tensor_walk(const __grid_cons
     bool ok = true;
     for (uint32_t it = 0; ok; ++it) {
       const uint32_t slot = it & 1u;
-      if (it >= 2u && !(ok = mbar_wait<1000>(smem_addr(&sh->seed_empty[slot]), ((it >> 1) - 1u) & 1u, give_up))) break;
-      if (part == 0 && lane == 0) {
-        const uint64_t first = (uint64_t)atomicAdd(a.work, 1u) * a.batch;
-        sh->first[slot] = first;
-        sh->count[slot] = first >= nunits ? 0u : (uint32_t)min((uint64_t)a.batch, nunits - first);
+      // the first seed warp takes the batch; the other one waits until it has.  It waits
+      // with a limit as every role does: the first may have left after a time-out.
+      // (A slot's next batch is taken only when both have filled this one, so that
+      // each phase of `taken` is seen.)
+      if (part == 0u) {
+        if (it >= 2u && !(ok = mbar_wait<1000>(smem_addr(&sh->seed_empty[slot]), ((it >> 1) - 1u) & 1u, give_up))) break;
+        if (lane == 0) {
+          const uint64_t first = (uint64_t)atomicAdd(a.work, 1u) * a.batch;
+          sh->first[slot] = first;
+          sh->count[slot] = first >= nunits ? 0u : (uint32_t)min((uint64_t)a.batch, nunits - first);
+          mbar_arrive(smem_addr(&sh->taken[slot]));
+        }
+        __syncwarp();
+      } else if (!(ok = mbar_wait<200>(smem_addr(&sh->taken[slot]), (it >> 1) & 1u, give_up))) {
+        break;
       }
-      asm volatile("bar.sync 1, 64;" ::: "memory");  // the two seed warps
       const uint32_t count = sh->count[slot];
       if (count) {
         const uint64_t vi = sh->first[slot] + (lane < count ? lane : 0u);
