@@ -140,6 +140,15 @@ int pps_debug_fail_allocs(int skip, int count);
    unchanged; only speed is.  Applies to every engine from the next call. */
 int pps_debug_limits(int warp_queue, uint32_t first_candidates);
 
+/* Test hook for the tensor walk's bounded waits: the warp that hands out the
+   work of each block stops before that block's `batch`-th batch (0, 1, ...; -1:
+   never, and the usual limit again) and waits for a flag that nothing sets,
+   until wait_clocks SM clocks have run out (1..8000000000).  Every other role
+   then leaves its waits too, the kernel ends by itself, and the call returns
+   PPS_ERR_TIMEOUT; the engine stays usable.  Applies to every engine from the
+   next call. */
+int pps_debug_tensor_stall(int batch, uint64_t wait_clocks);
+
 /* Apply the reference's option rules (main.c:916-931, main.c:971-972,
    pps/app.c:657-712, pps/appcu.cu:158-204, pps/appcu.cu:236). */
 int pps_normalize(const pps_job_spec *in, pps_job_params *out);

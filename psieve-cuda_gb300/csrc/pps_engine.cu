@@ -80,6 +80,24 @@ extern "C" int pps_debug_limits(int warp_queue, uint32_t first_candidates) {
   return PPS_OK;
 }
 
+static std::atomic<uint32_t> g_dbg_stall{~0u};
+static std::atomic<uint64_t> g_dbg_wait{0};
+
+// The batch before which the tensor walk's seeds stop (~0: none), and its wait limit in clocks (0: the usual one).
+static void debug_tensor_stall(uint32_t* at, long long* limit) {
+  *at = g_dbg_stall.load(std::memory_order_relaxed);
+  const uint64_t w = g_dbg_wait.load(std::memory_order_relaxed);
+  *limit = w ? (long long)w : TW_WAIT_LIMIT;
+}
+
+extern "C" int pps_debug_tensor_stall(int batch, uint64_t wait_clocks) {
+  if (batch >= 0 && (!wait_clocks || wait_clocks > (uint64_t)TW_WAIT_LIMIT))
+    return set_err(PPS_ERR_INVALID_PARAM, "a stall needs a wait limit of at most %lld clocks", TW_WAIT_LIMIT);
+  g_dbg_stall = batch < 0 ? ~0u : (uint32_t)batch;
+  g_dbg_wait = batch < 0 ? 0 : wait_clocks;
+  return PPS_OK;
+}
+
 extern "C" const char* pps_version(void) { return "ppsgpu-0.1 (sm_103a)"; }
 
 // ------------------------------------------------------------ normalize
@@ -753,6 +771,7 @@ int run_tensor_walk(pps_engine* e, const pps_job_params* jp, const TensorPlan& p
   a.work = e->counters.p + CNT_TENSOR;
   a.to = to;
   a.masks = e->masks.p;
+  debug_tensor_stall(&a.stall_at, &a.wait_limit);
   CU(launch_tensor_walk(a, e->num_sms, e->st, &e->launches));
   return PPS_OK;
 }

@@ -36,15 +36,18 @@ __device__ __forceinline__ void mbar_arrive_lane0(uint32_t bar, uint32_t count =
       "r"(count), "r"(threadIdx.x & 31u)
       : "memory");
 }
-// Waits for a phase of the barrier, with a limit: false when MBAR_LIMIT clocks
-// (about 4 s) ran out or another role of the CTA gave up (*give_up != 0, set
-// here on a time-out), so that every role then leaves its loops and the kernel
-// ends.  The votes keep the branches uniform.  PAUSE: ns to sleep between
-// attempts, for the roles that run ahead, so that their polling takes no issue
-// slots from the others.
-constexpr long long MBAR_LIMIT = 8000000000ll;
+// Waits for a phase of the barrier, with a limit: false when the bound's clocks
+// ran out or another role that shares it gave up (give_up != 0, set here on a
+// time-out), so that every role then leaves its loops and the kernel ends.  The
+// votes keep the branches uniform.  PAUSE: ns to sleep between attempts, for the
+// roles that run ahead, so that their polling takes no issue slots from the
+// others.
+struct MbarBound {  // in shared memory
+  long long limit;
+  uint32_t give_up;
+};
 template <uint32_t PAUSE>
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile uint32_t* give_up) {
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile MbarBound* bound) {
   if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
   const long long t0 = clock64();
 #pragma unroll 1
@@ -52,8 +55,8 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     if (PAUSE) __nanosleep(PAUSE);
     if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
     if ((i & 63u) == 0u) {
-      if (clock64() - t0 > MBAR_LIMIT) *give_up = 1u;
-      if (__any_sync(0xffffffffu, *give_up != 0u)) return false;
+      if (clock64() - t0 > bound->limit) bound->give_up = 1u;
+      if (__any_sync(0xffffffffu, bound->give_up != 0u)) return false;
     }
   }
 }

@@ -92,11 +92,14 @@ constexpr uint32_t SIDE_BIT = 0x80000000u;  // a twin candidate of the +1 side
 
 struct __align__(128) Shared {
   uint64_t seed_full[2], seed_empty[2], taken[2];
+  uint64_t never;     // nothing arrives (pps_debug_tensor_stall)
+  uint64_t drain[2];  // the MMAs of each half, at the end
   uint64_t ab_full[TW_STAGES], ab_empty[TW_STAGES];
   uint64_t d_full[TW_GROUPS], d_empty[TW_GROUPS / 2];
   uint64_t first[2];
   uint32_t count[2];   // units of the batch in this slot; 0: no more
-  uint32_t tmem, give_up;
+  MbarBound bound, late[2];  // of every wait; of the waits for `drain`
+  uint32_t tmem;
   uint64_t tab[2][32][TAB_PITCH];              // G_0..7, H_0..15, p, ps
 };
 
@@ -372,7 +375,7 @@ __global__ void __launch_bounds__(TW_THREADS, 1) k_tensor_walk(const __grid_cons
   const uint32_t ntiles = (nb + TW_TILE - 1) / TW_TILE, npairs = (ntiles + 1u) / 2u, nbp = ntiles * TW_TILE;
   unsigned char* const bop = smem_raw + sizeof(Shared);  // B operands: TW_STAGES x nbp rows x 32 B
   uint32_t* const S = reinterpret_cast<uint32_t*>(bop + TW_STAGES * nbp * 32u);
-  volatile uint32_t* const give_up = &sh->give_up;
+  volatile MbarBound* const bound = &sh->bound;
   if (tid == 0) {
     for (int i = 0; i < 2; ++i) {
       mbar_init(smem_addr(&sh->seed_full[i]), TW_SEED_WARPS);
@@ -387,7 +390,12 @@ __global__ void __launch_bounds__(TW_THREADS, 1) k_tensor_walk(const __grid_cons
       mbar_init(smem_addr(&sh->d_full[i]), 1);
       if (i < TW_GROUPS / 2) mbar_init(smem_addr(&sh->d_empty[i]), 8);
     }
-    sh->give_up = 0;
+    mbar_init(smem_addr(&sh->never), 1);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(smem_addr(&sh->drain[i]), 1);
+      sh->late[i] = MbarBound{TW_WAIT_LIMIT, 0u};
+    }
+    sh->bound = MbarBound{a.wait_limit, 0u};
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   // the last tile's rows beyond the unit's: no digits, and a constant slot of
@@ -423,7 +431,7 @@ __global__ void __launch_bounds__(TW_THREADS, 1) k_tensor_walk(const __grid_cons
     bool ok = true;
     for (uint32_t it = 0; ok; ++it) {
       const uint32_t slot = it & 1u;
-      if (!(ok = mbar_wait<200>(smem_addr(&sh->seed_full[slot]), (it >> 1) & 1u, give_up))) break;
+      if (!(ok = mbar_wait<200>(smem_addr(&sh->seed_full[slot]), (it >> 1) & 1u, bound))) break;
       const uint32_t count = sh->count[slot];
       if (!count) break;
       uint4* out = a.masks + sh->first[slot] * (ntiles * 4u) + (warp & 3u);
@@ -431,7 +439,7 @@ __global__ void __launch_bounds__(TW_THREADS, 1) k_tensor_walk(const __grid_cons
         for (; skip < npairs; skip += 2u) {
           const uint32_t t = 2u * skip + (group & 1u);
           if (t == ntiles) continue;  // a pair's only tile is the other group's
-          if (!(ok = mbar_wait<0>(full, par, give_up))) break;
+          if (!(ok = mbar_wait<0>(full, par, bound))) break;
           par ^= 1u;
           tc_fence_after();
           uint32_t q[32], m[4];
@@ -466,13 +474,13 @@ __global__ void __launch_bounds__(TW_THREADS, 1) k_tensor_walk(const __grid_cons
     bool ok = true;
     for (uint32_t it = 0; ok; ++it) {
       const uint32_t slot = it & 1u;
-      if (!(ok = mbar_wait<200>(smem_addr(&sh->seed_full[slot]), (it >> 1) & 1u, give_up))) break;
+      if (!(ok = mbar_wait<200>(smem_addr(&sh->seed_full[slot]), (it >> 1) & 1u, bound))) break;
       const uint32_t count = sh->count[slot];
       if (!count) break;
       for (uint32_t unit = 0; unit < count; ++unit, ++unit_no) {
         if (unit_no % TW_BGROUPS != group) continue;
         const uint32_t st = unit_no % TW_STAGES, use = unit_no / TW_STAGES;
-        if (use && !(ok = mbar_wait<100>(smem_addr(&sh->ab_empty[st]), (use - 1u) & 1u, give_up))) break;
+        if (use && !(ok = mbar_wait<100>(smem_addr(&sh->ab_empty[st]), (use - 1u) & 1u, bound))) break;
         const uint64_t* tab = sh->tab[slot][unit];
         const uint32_t* Sp = S + ((size_t)slot * 32u + unit) * pitch;
         uint4* b4 = reinterpret_cast<uint4*>(bop) + st * 2u * nbp;
@@ -532,7 +540,8 @@ __global__ void __launch_bounds__(TW_THREADS, 1) k_tensor_walk(const __grid_cons
       // (A slot's next batch is taken only when both have filled this one, so that
       // each phase of `taken` is seen.)
       if (part == 0u) {
-        if (it >= 2u && !(ok = mbar_wait<1000>(smem_addr(&sh->seed_empty[slot]), ((it >> 1) - 1u) & 1u, give_up))) break;
+        if (it == a.stall_at && !(ok = mbar_wait<1000>(smem_addr(&sh->never), 0u, bound))) break;
+        if (it >= 2u && !(ok = mbar_wait<1000>(smem_addr(&sh->seed_empty[slot]), ((it >> 1) - 1u) & 1u, bound))) break;
         if (lane == 0) {
           const uint64_t first = (uint64_t)atomicAdd(a.work, 1u) * a.batch;
           sh->first[slot] = first;
@@ -540,7 +549,7 @@ __global__ void __launch_bounds__(TW_THREADS, 1) k_tensor_walk(const __grid_cons
           mbar_arrive(smem_addr(&sh->taken[slot]));
         }
         __syncwarp();
-      } else if (!(ok = mbar_wait<200>(smem_addr(&sh->taken[slot]), (it >> 1) & 1u, give_up))) {
+      } else if (!(ok = mbar_wait<200>(smem_addr(&sh->taken[slot]), (it >> 1) & 1u, bound))) {
         break;
       }
       const uint32_t count = sh->count[slot];
@@ -621,18 +630,18 @@ __global__ void __launch_bounds__(TW_THREADS, 1) k_tensor_walk(const __grid_cons
     bool ok = true;
     for (uint32_t it = 0; ok; ++it) {
       const uint32_t slot = it & 1u;
-      if (!mbar_wait<0>(smem_addr(&sh->seed_full[slot]), (it >> 1) & 1u, give_up)) break;
+      if (!(ok = mbar_wait<0>(smem_addr(&sh->seed_full[slot]), (it >> 1) & 1u, bound))) break;
       const uint32_t count = __shfl_sync(0xffffffffu, *(volatile uint32_t*)&sh->count[slot], 0);
       if (!count) break;
       // this half's pairs of the batch's units, in order
       for (uint32_t unit = 0; unit < count && ok; ++unit, ++unit_no) {
         const uint32_t st = unit_no % TW_STAGES;
-        if (!(ok = mbar_wait<0>(abf0 + st * 8u, (unit_no / TW_STAGES) & 1u, give_up))) break;
+        if (!(ok = mbar_wait<0>(abf0 + st * 8u, (unit_no / TW_STAGES) & 1u, bound))) break;
         const uint32_t atm = TW_ACOL + st * 16u, b_st = b_lo + st * nbp * 2u;
         if (skip >= npairs) mbar_arrive_lane0(abe0 + st * 8u);  // a unit of one pair, the other half's
         else {
           for (; skip < npairs; skip += 2u) {
-            if (!(ok = mbar_wait<0>(empty, free_par, give_up))) break;
+            if (!(ok = mbar_wait<0>(empty, free_par, bound))) break;
             free_par ^= 1u;
             tc_fence_after();
             const uint32_t b = b_st + 2u * skip * TW_TILE;
@@ -645,15 +654,23 @@ __global__ void __launch_bounds__(TW_THREADS, 1) k_tensor_walk(const __grid_cons
       }
       if (ok && lane == 0) mbar_arrive(smem_addr(&sh->seed_empty[slot]));
     }
-    // every arrival has come before the block ends
-    if (ok && unit_no) mbar_wait<0>(abe0 + (unit_no - 1u) % TW_STAGES * 8u, ((unit_no - 1u) / TW_STAGES) & 1u, give_up);
+    // Nothing may reach this block's memory after it ended.  The arrivals of the
+    // commits: the test warps have seen those of the tiles, here each stage's last
+    // use is waited for (with one pair of tiles to a unit the halves take units in
+    // turn, and the last unit's stage says nothing of the other half's).  After a
+    // time-out those may never come, but what was issued ends: a last commit, and a
+    // wait that does not heed the others' time-outs.
+    for (uint32_t i = 1; ok && i <= min(TW_STAGES, unit_no); ++i)
+      ok = mbar_wait<0>(abe0 + (unit_no - i) % TW_STAGES * 8u, ((unit_no - i) / TW_STAGES) & 1u, bound);
+    mma_commit(smem_addr(&sh->drain[half]));
+    mbar_wait<0>(smem_addr(&sh->drain[half]), 0u, &sh->late[half]);
   }
   __syncwarp();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   if (warp == 0) tmem_dealloc(tmem, 512);
-  if (tid == 0 && sh->give_up) a.work[2] = 1u;
+  if (tid == 0 && (sh->bound.give_up | sh->late[0].give_up | sh->late[1].give_up)) a.work[2] = 1u;
 }
 
 size_t tensor_smem(uint32_t nb, uint32_t pitch) {

@@ -47,11 +47,14 @@ struct TensorArgs {
   uint32_t* work;        // [0] batches taken (zeroed before each launch)
                          // [1] set when a prime outside [pmin, pmax) was met (not walked)
                          // [2] set when a bounded wait ran out
+  long long wait_limit;  // clocks that a wait may take
+  uint32_t stall_at;     // batch of each CTA before which the seeds stop (pps_debug_tensor_stall; ~0: none)
   uint4* masks;          // which rows pass: of each unit, tile and 32 rows a bit per row for columns 0-31,
                          // 32-63, 64-95 and 96-111 of the tile
   TensorHits to;
 };
 
+constexpr long long TW_WAIT_LIMIT = 8000000000ll;  // clocks: about 4 s
 constexpr double TW_LEAST_COST = 635.0;      // of one unit (TensorPlan::cost)
 constexpr uint32_t TW_MAX_MASKS = 1u << 24;  // 268 MB; their numbers have 25 bits in k_tensor_check
 

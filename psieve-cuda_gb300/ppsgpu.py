@@ -205,6 +205,7 @@ def load(path: str | os.PathLike | None = None) -> ctypes.CDLL:
         "pps_version": (ctypes.c_char_p, []),
         "pps_debug_fail_allocs": (ctypes.c_int, [ctypes.c_int, ctypes.c_int]),
         "pps_debug_limits": (ctypes.c_int, [ctypes.c_int, ctypes.c_uint32]),
+        "pps_debug_tensor_stall": (ctypes.c_int, [ctypes.c_int, ctypes.c_uint64]),
         "pps_normalize": (ctypes.c_int, [P(JobSpec), P(JobParams)]),
         "pps_engine_create": (ctypes.c_int, [ctypes.c_int, P(ctypes.c_void_p)]),
         "pps_engine_destroy": (None, [ctypes.c_void_p]),
