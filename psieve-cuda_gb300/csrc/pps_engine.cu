@@ -847,10 +847,11 @@ extern "C" int pps_engine_set_input(pps_engine* e, const pps_input* in) {
 }
 
 // The tensor walk's status words in the pinned copy of the counters: an error
-// where a bounded wait ran out; *outside is set where the caller's list held a
+// where a launch failed; *outside is set where the caller's list held a
 // prime outside the job's range (that walk leaves it out).
 int tensor_status(const pps_engine* e, bool* outside) {
   const uint32_t* c = (const uint32_t*)e->h_pinned + CNT_TENSOR;
+  if (c[2] == TW_BAD_TMEM) return set_err(PPS_ERR_CUDA, "tensor walk: tensor memory does not start at 0");
   if (c[2]) return set_err(PPS_ERR_TIMEOUT, "tensor walk: a bounded device wait expired");
   if (c[1] && outside) *outside = true;
   return PPS_OK;

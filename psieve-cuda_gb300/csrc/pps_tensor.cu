@@ -99,7 +99,7 @@ struct __align__(128) Shared {
   uint64_t first[2];
   uint32_t count[2];   // units of the batch in this slot; 0: no more
   MbarBound bound, late[2];  // of every wait; of the waits for `drain`
-  uint32_t tmem;
+  uint32_t tmem, failed;
   uint64_t tab[2][32][TAB_PITCH];              // G_0..7, H_0..15, p, ps
 };
 
@@ -321,6 +321,7 @@ __device__ __forceinline__ void check_row(const TensorArgs& a, bool live, uint32
 template <bool TWIN, bool LONG>
 __global__ void __launch_bounds__(256) k_tensor_check(const __grid_constant__ TensorArgs a, uint32_t n, uint32_t ntiles) {
   __shared__ uint32_t queue[8][64];
+  if (a.work[2]) return;  // the masks are not all written
   uint32_t* const q = queue[threadIdx.x >> 5];
   const uint32_t lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
   uint32_t have = 0;
@@ -396,6 +397,7 @@ __global__ void __launch_bounds__(TW_THREADS, 1) k_tensor_walk(const __grid_cons
       sh->late[i] = MbarBound{TW_WAIT_LIMIT, 0u};
     }
     sh->bound = MbarBound{a.wait_limit, 0u};
+    sh->failed = a.work[2];
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   // the last tile's rows beyond the unit's: no digits, and a constant slot of
@@ -411,11 +413,12 @@ __global__ void __launch_bounds__(TW_THREADS, 1) k_tensor_walk(const __grid_cons
   __syncthreads();
   tc_fence_after();
   // All of TMEM is this CTA's (it fills the SM), so it starts at 0: a constant in
-  // the addresses below, checked here.
+  // the addresses below, checked here.  After an error of an earlier launch of the
+  // call there is nothing left to do.
   const uint32_t tmem = 0;
-  if (sh->tmem != tmem) {
+  if (sh->tmem != tmem || sh->failed) {
     if (warp == 0) tmem_dealloc(sh->tmem, 512);
-    if (tid == 0) a.work[2] = 1u;
+    if (tid == 0 && !sh->failed) a.work[2] = TW_BAD_TMEM;
     return;
   }
 
@@ -670,7 +673,7 @@ __global__ void __launch_bounds__(TW_THREADS, 1) k_tensor_walk(const __grid_cons
   __syncthreads();
   tc_fence_after();
   if (warp == 0) tmem_dealloc(tmem, 512);
-  if (tid == 0 && (sh->bound.give_up | sh->late[0].give_up | sh->late[1].give_up)) a.work[2] = 1u;
+  if (tid == 0 && (sh->bound.give_up | sh->late[0].give_up | sh->late[1].give_up)) a.work[2] = TW_TIMED_OUT;
 }
 
 size_t tensor_smem(uint32_t nb, uint32_t pitch) {

@@ -46,7 +46,7 @@ struct TensorArgs {
   uint32_t batch;        // units a CTA takes at a time (1..32)
   uint32_t* work;        // [0] batches taken (zeroed before each launch)
                          // [1] set when a prime outside [pmin, pmax) was met (not walked)
-                         // [2] set when a bounded wait ran out
+                         // [2] set when a launch failed: TW_TIMED_OUT, TW_BAD_TMEM
   long long wait_limit;  // clocks that a wait may take
   uint32_t stall_at;     // batch of each CTA before which the seeds stop (pps_debug_tensor_stall; ~0: none)
   uint4* masks;          // which rows pass: of each unit, tile and 32 rows a bit per row for columns 0-31,
@@ -54,6 +54,8 @@ struct TensorArgs {
   TensorHits to;
 };
 
+constexpr uint32_t TW_TIMED_OUT = 1u;  // a bounded wait ran out
+constexpr uint32_t TW_BAD_TMEM = 2u;   // tensor memory did not start at 0
 constexpr long long TW_WAIT_LIMIT = 8000000000ll;  // clocks: about 4 s
 constexpr double TW_LEAST_COST = 635.0;      // of one unit (TensorPlan::cost)
 constexpr uint32_t TW_MAX_MASKS = 1u << 24;  // 268 MB; their numbers have 25 bits in k_tensor_check

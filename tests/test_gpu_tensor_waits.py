@@ -4,6 +4,8 @@ batch and waits, with a short limit, for a flag that nothing sets
 PPS_ERR_TIMEOUT, and the same engine then gives the exact result."""
 from __future__ import annotations
 
+import time
+
 import pytest
 
 pytestmark = pytest.mark.gpu
@@ -47,6 +49,27 @@ def test_a_wait_that_runs_out(pps, stall, pmin, span, kmax, sign, batch):
         stall(-1)
         got, again = eng.run_job(jp)
         assert got.tobytes() == want.tobytes() and again.raw_hits == st.raw_hits and again.primes == st.primes
+
+
+def test_one_wait_runs_out_not_one_a_part(pps):
+    """A job of three parts: after the first part's time-out the other launches
+    return at once, so the call takes one wait limit, not three."""
+    clocks = 1_000_000_000  # about half a second
+    jp = pps.normalize(pmin=42 * 10**12, pmax=42 * 10**12 + 75 * 10**6, kmin=1201, kmax=9999, nmin=2_000_000,
+                       nmax=3_000_000)
+    with pps.Engine(0) as eng:
+        eng.set_variant(31)
+        eng.run_job(jp)
+        lib = pps.load()
+        try:
+            assert lib.pps_debug_tensor_stall(0, clocks) == pps.PPS_OK
+            t0 = time.perf_counter()
+            with pytest.raises(pps.PPSError) as ei:
+                eng.run_job(jp)
+            took = time.perf_counter() - t0
+        finally:
+            lib.pps_debug_tensor_stall(-1, 0)
+        assert ei.value.code == pps.PPS_ERR_TIMEOUT and took < 1.0
 
 
 def test_the_stall_needs_a_limit(pps):
