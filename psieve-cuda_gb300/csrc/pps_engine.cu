@@ -232,6 +232,7 @@ extern "C" int pps_engine_create(int device, pps_engine** out) {
     cudaDeviceProp prop;
     if (cudaGetDeviceProperties(&prop, device) != cudaSuccess) { rc = set_err(PPS_ERR_CUDA, "cudaGetDeviceProperties failed"); break; }
     e->num_sms = prop.multiProcessorCount;
+    if (tensor_setup() != cudaSuccess) { rc = set_err(PPS_ERR_CUDA, "tensor walk: shared memory"); break; }
     if (cudaStreamCreateWithFlags(&e->st, cudaStreamNonBlocking) != cudaSuccess) { rc = set_err(PPS_ERR_CUDA, "stream"); break; }
     for (auto& v : e->ev)
       if (cudaEventCreate(&v) != cudaSuccess) { rc = set_err(PPS_ERR_CUDA, "event"); break; }

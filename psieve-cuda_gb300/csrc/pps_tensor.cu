@@ -734,14 +734,20 @@ size_t tensor_masks(const TensorPlan& plan, uint64_t np) {
   return (size_t)std::min<uint64_t>(np * plan.units * tiles_of(plan) * 4u, TW_MAX_MASKS);
 }
 
+cudaError_t tensor_setup() {
+  cudaError_t e = cudaSuccess;
+  for (auto fn : {k_tensor_walk<4>, k_tensor_walk<5>})
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TW_MAX_SMEM);
+  return e;
+}
+
 cudaError_t launch_tensor_walk(TensorArgs a, int num_sms, cudaStream_t st, uint64_t* launches) {
   auto fn = a.plan.digits == 4u ? k_tensor_walk<4> : k_tensor_walk<5>;
   const bool twin = a.side == 2u, lng = a.plan.s > 32u;
   auto check = twin ? (lng ? k_tensor_check<true, true> : k_tensor_check<true, false>)
                     : (lng ? k_tensor_check<false, true> : k_tensor_check<false, false>);
   const size_t smem = tensor_smem(a.plan.nb, a.plan.pitch);
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
+  cudaError_t e;
   const uint32_t ntiles = tiles_of(a.plan);
   uint64_t part = TW_MAX_MASKS / (a.plan.units * ntiles * 4u);  // primes of one part
   const uint64_t np = a.np, nparts = (np + part - 1) / part;

@@ -62,6 +62,11 @@ constexpr uint32_t TW_MAX_MASKS = 1u << 24;  // 268 MB; their numbers have 25 bi
 
 // Masks for np primes, or for one part of them.
 size_t tensor_masks(const TensorPlan& plan, uint64_t np);
+// Once for a device, before its first walk: lets the kernels have all the shared
+// memory that a plan may ask for.  (The setting is the device's and not a
+// launch's: set to each job's size, one thread's smaller job would make another's
+// launches fail.)
+cudaError_t tensor_setup();
 // The walk and the re-check of np primes, in parts of TW_MAX_MASKS masks.  *launches += the kernels launched.
 cudaError_t launch_tensor_walk(TensorArgs a, int num_sms, cudaStream_t st, uint64_t* launches);
 
