@@ -19,18 +19,22 @@
 // the low 16 bits of each f32 accumulator are the fraction itself, in units of
 // 2^-16 (base 32: 2^-15), and the test is an unsigned 16-bit compare.
 //
-// Exactness.  The test never rejects a hit; what it passes (about 1 in 2,000)
-// is recomputed exactly, and only those values give candidates.  Errors of the
-// tested fraction, in 2^-16:
-//   - h products are whole multiples of 2^-12, exact in the accumulator; the l
-//     sum enters as the accumulator of the h MMA, truncated to its last bit
-//     (1; base 32: 2) and, measured on the GB300, each product at a quarter of
-//     it, which no h product reaches;
+// Exactness.  The test never rejects a hit, if the accumulator works as said
+// below; what it passes (about 1 in 2,000) is recomputed exactly, and only those
+// values give candidates.  Errors of the tested fraction, in 2^-16 (base 32 in
+// brackets; tests/test_tensor_margins.py has a model of them):
+//   - l: rounded to 24 bits (2^-14 of 2^-12 at most) and to fp16 (2^-13), in each
+//     of 15 slots with digits up to 8 (16), and K_a beyond 32 bits (2^-16 a digit):
+//     0.36 (0.71) either way.  h products are whole multiples of 2^-12, exact;
+//   - the accumulator's last bit, 1 (2): the l sum is cut towards zero to a quarter
+//     of it, which raises a negative one by up to 0.25 (0.5), and the whole, which
+//     is positive, is cut to it, which lowers it by less than 1 (2).  The quarter is
+//     measured on the GB300 and in no manual; below it does not matter;
 //   - v_b beyond the 15 digits: K_a, in (-p/2, p/2), times half a unit of the
-//     last digit, p 2^-62 (base 32: p 2^-77);
-//   - l beyond its 11 bits, K_a beyond 32 bits: below 0.1 together.
+//     last digit, p 2^-62 (base 32: p 2^-77), either way;
+//   - base 32: doubling a pair of fractions moves a bit into the upper one: (1) up.
 // `off` shifts the fraction so that the smallest hit stays above zero, and
-// `thr` is eps plus both errors (tensor_plan).
+// `thr` is eps plus the errors either way (tensor_plan).
 //
 // One CTA per SM, its warps in roles (mbarriers between them):
 //   2 seed warps    batch of 32 units, lane = unit: the expansion S, the
@@ -692,9 +696,10 @@ bool tensor_plan(const pps_job_params* jp, TensorPlan* out) {
   if (jp->pmax <= jp->pmin || jp->kmax < jp->kmin) return false;
   const uint32_t g = jp->pmax <= (1ull << 47) ? 4u : 5u;
   const uint64_t N = jp->nmax - jp->nmin;
-  // errors in 2^-16, see the head of this file: p beyond the digits, the accumulator's last bit
+  // errors in 2^-16, see the head of this file: v_b's, l's, the accumulator's, the doubling's
   const double tail = ldexp((double)jp->pmax, g == 4u ? 16 - 62 : 16 - 77);
-  const double below = tail + (g == 4u ? 1.4 : 3.4), above = tail + (g == 4u ? 0.4 : 1.7);
+  const double below = tail + (g == 4u ? 0.36 + 1.0 : 0.71 + 2.0);
+  const double above = tail + (g == 4u ? 0.36 + 0.25 : 0.71 + 0.5 + 1.0);
   const double one = (double)jp->kmax / (double)jp->pmin * 65536.0;  // eps at s = 1
   bool found = false;
   for (uint64_t units = 1; units <= 4096 && (!found || (double)units * TW_LEAST_COST < out->cost); units *= 2) {
