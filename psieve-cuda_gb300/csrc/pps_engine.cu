@@ -754,12 +754,14 @@ static double job_primes(const pps_engine* e, const pps_job_params* jp) {
 }
 
 int run_tensor_walk(pps_engine* e, const pps_job_params* jp, const TensorPlan& plan, const uint64_t* dP,
-                    const uint64_t* dPinv, uint64_t np, const TensorHits& to) {
+                    const uint64_t* dPinv, uint64_t np, const TensorHits& to, bool caller_list) {
   if (int rc = e->masks.ensure(tensor_masks(plan, np))) return rc;
   TensorArgs a;
   a.P = dP;
   a.Pinv = dPinv;
   a.np = np;
+  a.list = dP;
+  a.listed = caller_list ? np : 0;
   a.pmin = jp->pmin;
   a.pmax = jp->pmax;
   a.kmin = jp->kmin;
@@ -854,7 +856,8 @@ int tensor_status(const pps_engine* e, bool* outside) {
   const uint32_t* c = (const uint32_t*)e->h_pinned + CNT_TENSOR;
   if (c[2] == TW_BAD_TMEM) return set_err(PPS_ERR_CUDA, "tensor walk: tensor memory does not start at 0");
   if (c[2]) return set_err(PPS_ERR_TIMEOUT, "tensor walk: a bounded device wait expired");
-  if (c[1] && outside) *outside = true;
+  if (c[1] && !outside) return set_err(PPS_ERR_INVALID_PARAM, "tensor walk: a prime outside the job's p range");
+  if (c[1]) *outside = true;
   return PPS_OK;
 }
 
@@ -1054,11 +1057,13 @@ extern "C" int pps_run_job(pps_engine* e, const pps_job_params* jp, pps_factor* 
   return set_err(PPS_ERR_INSUFFICIENT_RESOURCE, "hit buffer overflow persisted");
 }
 
-// Walk primes already on the device; hits accumulate in e->hits.  in_range: the
-// primes lie in [pmin, pmax), or the tensor walk, which needs that, has not
-// found otherwise yet.
-static int walk_device_list(pps_engine* e, const pps_job_params* jp, const uint64_t* dP, size_t np,
+// Walk primes already on the device (or page-locked: then *dP becomes the
+// device copy that the tensor walk takes); hits accumulate in e->hits.  in_range:
+// the tensor walk, which needs the primes to lie in [pmin, pmax), has not found
+// otherwise yet.
+static int walk_device_list(pps_engine* e, const pps_job_params* jp, const uint64_t** d_list, size_t np,
                             pps_job_stats* st, bool in_range, bool* is_tensor) {
+  const uint64_t*& dP = *d_list;
   TensorPlan plan;
   const bool tensor = in_range && tensor_choice(e, jp, (double)np, &plan);
   *is_tensor = tensor;
@@ -1070,8 +1075,6 @@ static int walk_device_list(pps_engine* e, const pps_job_params* jp, const uint6
   if (split < 0) return split;
   if (st) st->split = (uint32_t)split;
   CU(cudaEventRecord(e->ev[2], e->st));
-  if (tensor)
-    CU(cudaMemsetAsync(e->counters.p + CNT_TENSOR, 0, (CNT_WORDS - CNT_TENSOR) * sizeof(uint32_t), e->st));
   cudaPointerAttributes at;
   if (tensor && cudaPointerGetAttributes(&at, dP) == cudaSuccess && at.type == cudaMemoryTypeHost) {
     // a page-locked list: its re-check would read some primes a few times more
@@ -1079,7 +1082,7 @@ static int walk_device_list(pps_engine* e, const pps_job_params* jp, const uint6
     CU(cudaMemcpyAsync(e->P.p, dP, np * sizeof(uint64_t), cudaMemcpyDefault, e->st));
     dP = e->P.p;
   }
-  const int rc = tensor ? run_tensor_walk(e, jp, plan, dP, nullptr, np, job_hits(e))
+  const int rc = tensor ? run_tensor_walk(e, jp, plan, dP, nullptr, np, job_hits(e), true)
                         : run_walk(e, jp, variant, dP, nullptr, nullptr, np, 0, 0, (uint32_t)split);
   if (rc) return rc;
   CU(cudaEventRecord(e->ev[3], e->st));
@@ -1107,9 +1110,9 @@ extern "C" int pps_check_primes_device(pps_engine* e, const pps_job_params* jp, 
     if (rc) return rc;
     e->hit_cap_limit = attempt == 0 ? debug_first_hit_cap() : 0;
     if (st) memset(st, 0, sizeof *st);
-    CU(cudaMemsetAsync(e->counters.p, 0, 2 * sizeof(uint32_t), e->st));
+    CU(cudaMemsetAsync(e->counters.p, 0, CNT_WORDS * sizeof(uint32_t), e->st));
     bool tensor = false, overflow = false, outside = false;
-    if (np && (rc = walk_device_list(e, jp, d_P, np, st, in_range, &tensor))) return rc;
+    if (np && (rc = walk_device_list(e, jp, &d_P, np, st, in_range, &tensor))) return rc;
     uint32_t raw = 0;
     rc = finish_job(e, jp, out, cap, nout, st, &raw, &overflow, tensor, &outside);
     if (st) st->raw_hits = raw;
@@ -1178,9 +1181,9 @@ extern "C" int pps_check_primes_raw(pps_engine* e, const pps_job_params* jp, con
   for (int attempt = 0; attempt < 4; ++attempt) {
     if ((rc = ensure_hit_buffers(e, hit_cap, std::max<size_t>(1u << 18, e->factors.n)))) return rc;
     e->hit_cap_limit = attempt == 0 ? debug_first_hit_cap() : 0;
-    CU(cudaMemsetAsync(e->counters.p, 0, 2 * sizeof(uint32_t), e->st));
+    CU(cudaMemsetAsync(e->counters.p, 0, CNT_WORDS * sizeof(uint32_t), e->st));
     bool tensor = false, outside = false;
-    if (np && (rc = walk_device_list(e, jp, dP, np, nullptr, in_range, &tensor))) return rc;
+    if (np && (rc = walk_device_list(e, jp, &dP, np, nullptr, in_range, &tensor))) return rc;
     CU(cudaMemcpyAsync(e->h_pinned, e->counters.p, (tensor ? CNT_WORDS : 1u) * sizeof(uint32_t),
                        cudaMemcpyDeviceToHost, e->st));
     CU(cudaStreamSynchronize(e->st));

@@ -325,7 +325,8 @@ __device__ __forceinline__ void check_row(const TensorArgs& a, bool live, uint32
 template <bool TWIN, bool LONG>
 __global__ void __launch_bounds__(256) k_tensor_check(const __grid_constant__ TensorArgs a, uint32_t n, uint32_t ntiles) {
   __shared__ uint32_t queue[8][64];
-  if (a.work[2]) return;  // the masks are not all written
+  if (a.work[1] | a.work[2]) return;  // the masks are not all written
+  if (blockIdx.x == 0 && threadIdx.x == 0) a.work[0] = 0;  // for the next walk
   uint32_t* const q = queue[threadIdx.x >> 5];
   const uint32_t lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
   uint32_t have = 0;
@@ -353,6 +354,23 @@ __global__ void __launch_bounds__(256) k_tensor_check(const __grid_constant__ Te
     }
   }
   if (have) check_row<TWIN, LONG>(a, lane < have, q[lane < have ? lane : 0u] >> 7, q[lane < have ? lane : 0u] & 127u, ntiles);
+}
+
+// A caller's list is looked at before its walk: work[1] is set where a prime is
+// not in [pmin, pmax), so that a list that is not for the tensor walk costs that
+// and not a walk more.  Up to TW_SCAN primes each block of the walk does it beside
+// its set-up (a launch less, 3 us of a call of 1,000 primes); of more, a kernel of
+// its own does (300,000 primes: 3 us of 1.52 ms).
+__device__ __forceinline__ bool any_outside(const TensorArgs& a, uint64_t i, uint64_t stride) {
+  bool out = false;
+#pragma unroll 4
+  for (; i < a.listed; i += stride) out |= a.list[i] - a.pmin >= a.pmax - a.pmin;
+  if (out) a.work[1] = 1u;
+  return out;
+}
+
+__global__ void __launch_bounds__(256) k_tensor_range(const __grid_constant__ TensorArgs a) {
+  any_outside(a, blockIdx.x * 256ull + threadIdx.x, gridDim.x * 256ull);
 }
 
 // Both 16-bit minima of 8 and of 16 registers.
@@ -401,7 +419,7 @@ __global__ void __launch_bounds__(TW_THREADS, 1) k_tensor_walk(const __grid_cons
       sh->late[i] = MbarBound{TW_WAIT_LIMIT, 0u};
     }
     sh->bound = MbarBound{a.wait_limit, 0u};
-    sh->failed = a.work[2];
+    sh->failed = a.work[1] | a.work[2];
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   // the last tile's rows beyond the unit's: no digits, and a constant slot of
@@ -416,13 +434,17 @@ __global__ void __launch_bounds__(TW_THREADS, 1) k_tensor_walk(const __grid_cons
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  if (a.listed) {
+    if (any_outside(a, tid, TW_THREADS)) sh->failed = 1u;
+    __syncthreads();
+  }
   // All of TMEM is this CTA's (it fills the SM), so it starts at 0: a constant in
   // the addresses below, checked here.  After an error of an earlier launch of the
-  // call there is nothing left to do.
+  // call, or with a list that is not for this walk, there is nothing to do.
   const uint32_t tmem = 0;
   if (sh->tmem != tmem || sh->failed) {
+    if (tid == 0 && sh->tmem != tmem) a.work[2] = TW_BAD_TMEM;
     if (warp == 0) tmem_dealloc(sh->tmem, 512);
-    if (tid == 0 && !sh->failed) a.work[2] = TW_BAD_TMEM;
     return;
   }
 
@@ -752,7 +774,11 @@ cudaError_t launch_tensor_walk(TensorArgs a, int num_sms, cudaStream_t st, uint6
   auto check = twin ? (lng ? k_tensor_check<true, true> : k_tensor_check<true, false>)
                     : (lng ? k_tensor_check<false, true> : k_tensor_check<false, false>);
   const size_t smem = tensor_smem(a.plan.nb, a.plan.pitch);
-  cudaError_t e;
+  if (a.listed > TW_SCAN) {
+    k_tensor_range<<<8u * (uint32_t)num_sms, 256, 0, st>>>(a);
+    a.listed = 0;
+    ++*launches;
+  }
   const uint32_t ntiles = tiles_of(a.plan);
   uint64_t part = TW_MAX_MASKS / (a.plan.units * ntiles * 4u);  // primes of one part
   const uint64_t np = a.np, nparts = (np + part - 1) / part;
@@ -771,11 +797,10 @@ cudaError_t launch_tensor_walk(TensorArgs a, int num_sms, cudaStream_t st, uint6
     a.batch = (uint32_t)(batch < 32 ? batch : 32);
     const uint64_t nbatch = (units + a.batch - 1) / a.batch;
     const int grid = (int)std::min<uint64_t>(nbatch, (uint64_t)num_sms);
-    if ((e = cudaMemsetAsync(a.work, 0, sizeof(uint32_t), st)) != cudaSuccess) return e;
     fn<<<grid, TW_THREADS, smem, st>>>(a);
     const uint32_t masks = (uint32_t)units * ntiles * 4u;
     check<<<(int)std::min<uint32_t>((masks + 255u) / 256u, 8u * (uint32_t)num_sms), 256, 0, st>>>(a, masks, ntiles);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if (cudaError_t e = cudaGetLastError()) return e;
     *launches += 2;
   }
   return cudaSuccess;

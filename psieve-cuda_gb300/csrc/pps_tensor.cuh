@@ -39,13 +39,16 @@ struct TensorArgs {
   const uint64_t* P;
   const uint64_t* Pinv;  // or null: computed
   uint64_t np;
+  const uint64_t* list;  // a caller's list, whose primes may lie outside [pmin, pmax)
+  uint64_t listed;       // its length (0: the primes are known to lie inside)
   uint64_t pmin, pmax, kmin, kmax;
   uint32_t nmin, nmax;
   uint32_t side;         // 1: K = -2^-n (Proth), 0: K = 2^-n (Riesel), 2: both (twin)
   TensorPlan plan;
   uint32_t batch;        // units a CTA takes at a time (1..32)
-  uint32_t* work;        // [0] batches taken (zeroed before each launch)
-                         // [1] set when a prime outside [pmin, pmax) was met (not walked)
+  uint32_t* work;        // zeroed before a call's first launch
+                         // [0] batches taken (the re-check zeroes it again)
+                         // [1] set when a prime outside [pmin, pmax) was met: nothing more is walked
                          // [2] set when a launch failed: TW_TIMED_OUT, TW_BAD_TMEM
   long long wait_limit;  // clocks that a wait may take
   uint32_t stall_at;     // batch of each CTA before which the seeds stop (pps_debug_tensor_stall; ~0: none)
@@ -57,6 +60,7 @@ struct TensorArgs {
 constexpr uint32_t TW_TIMED_OUT = 1u;  // a bounded wait ran out
 constexpr uint32_t TW_BAD_TMEM = 2u;   // tensor memory did not start at 0
 constexpr long long TW_WAIT_LIMIT = 8000000000ll;  // clocks: about 4 s
+constexpr uint64_t TW_SCAN = 16384;    // of a list: 16 primes a thread of each block
 constexpr double TW_LEAST_COST = 635.0;      // of one unit (TensorPlan::cost)
 constexpr uint32_t TW_MAX_MASKS = 1u << 24;  // 268 MB; their numbers have 25 bits in k_tensor_check
 
@@ -77,7 +81,7 @@ cudaError_t launch_tensor_walk(TensorArgs a, int num_sms, cudaStream_t st, uint6
 bool tensor_choice(const pps_engine* e, const pps_job_params* jp, double np, pps::TensorPlan* plan,
                    double* saved = nullptr);
 int run_tensor_walk(pps_engine* e, const pps_job_params* jp, const pps::TensorPlan& plan, const uint64_t* dP,
-                    const uint64_t* dPinv, uint64_t np, const pps::TensorHits& to);
+                    const uint64_t* dPinv, uint64_t np, const pps::TensorHits& to, bool caller_list = false);
 // The status words in the pinned copy of the counters: an error if a wait ran
 // out, *outside if a prime was outside the job's range.
 int tensor_status(const pps_engine* e, bool* outside);

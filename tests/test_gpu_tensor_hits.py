@@ -184,3 +184,34 @@ def test_batch_jobs_with_hits_leave_for_the_tensor_walk(pps):
     (launches, waves, *got), (alone, waves0, *want) = runs
     assert waves == waves0 == 1 and launches == alone + 2 * 4
     assert got == want and all(len(f) for f in got[0][:4])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("where", [0, -1])
+def test_a_list_with_one_prime_outside_is_walked_once(pps, engine, where):
+    """One prime outside the job's range, first or last of 300,000: the call takes
+    what the recurrence alone takes, not that and a tensor walk."""
+    import time
+
+    spec = dict(pmin=42 * 10**12, pmax=42 * 10**12 + 10**7, kmin=3, kmax=9999, nmin=12_345, nmax=1_012_345)
+    jp = pps.normalize(**spec)
+    primes = engine.sieve_range(jp.pmin, jp.pmax, want_primes=True, cap=400_000)[0][:300_000].copy()
+    assert engine.check_primes(jp, primes)[1].variant == 31
+    primes[where] = 45 * 10**12 + 1
+
+    def best():
+        took = []
+        for _ in range(9):
+            t0 = time.perf_counter()
+            _, st = engine.check_primes(jp, primes)
+            took.append(time.perf_counter() - t0)
+        return min(took), st.variant
+
+    once, variant = best()
+    assert variant != 31
+    engine.set_variant(variant)
+    try:
+        alone, _ = best()
+    finally:
+        engine.set_variant(-1)
+    assert once < 1.2 * alone, (once, alone)
