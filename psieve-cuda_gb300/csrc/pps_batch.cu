@@ -1179,7 +1179,8 @@ int batch_set_jobs(pps_engine* e, uint32_t slot0, const pps_job_params* jobs, si
     double saved = 0;
     b->tensor.erase((uint32_t)(slot0 + j));
     if (!e->forced_bwalk && tensor_choice(e, &jobs[j], 0, &t.plan, &saved) &&
-        saved * (double)(jobs[j].pmax - jobs[j].pmin) > TENSOR_LEAST_SAVED * log((double)jobs[j].pmin)) {
+        saved * (double)(jobs[j].pmax - jobs[j].pmin) > TENSOR_LEAST_SAVED * log((double)jobs[j].pmin) &&
+        ensure_masks(e, t.plan, 32ull * e->num_sms) == PPS_OK) {  // (a wave's walks then have room, in parts)
       t.job = jobs[j];
       J.tensor = 1;
       b->tensor[(uint32_t)(slot0 + j)] = t;

@@ -753,9 +753,28 @@ static double job_primes(const pps_engine* e, const pps_job_params* jp) {
   return (double)std::min(jp->pmax - jp->pmin, e->batch_span) / log((double)jp->pmin);
 }
 
+// The tensor walk's masks for np primes or, where device memory is short, for a
+// part of them at a time, down to one batch of 32 units to each SM (below that
+// the launches would cost more than the recurrence).
+int ensure_masks(pps_engine* e, const TensorPlan& plan, uint64_t np) {
+  const uint64_t few = 32ull * e->num_sms / plan.units + 1;
+  const size_t least = tensor_masks(plan, std::min(np, few));
+  for (size_t n = tensor_masks(plan, np); n > e->masks.n; n = std::max(n / 4, least)) {
+    const int rc = e->masks.ensure(n, TW_MAX_MASKS);
+    if (rc && n == least) return rc;
+  }
+  return PPS_OK;
+}
+
+// As tensor_choice, with room for its masks: without, the recurrence walks, which
+// needs none.
+static bool tensor_takes(pps_engine* e, const pps_job_params* jp, double np, TensorPlan* plan) {
+  return tensor_choice(e, jp, np, plan) && ensure_masks(e, *plan, (uint64_t)np) == PPS_OK;
+}
+
 int run_tensor_walk(pps_engine* e, const pps_job_params* jp, const TensorPlan& plan, const uint64_t* dP,
                     const uint64_t* dPinv, uint64_t np, const TensorHits& to, bool caller_list) {
-  if (int rc = e->masks.ensure(tensor_masks(plan, np))) return rc;
+  if (int rc = ensure_masks(e, plan, np)) return rc;
   TensorArgs a;
   a.P = dP;
   a.Pinv = dPinv;
@@ -774,6 +793,7 @@ int run_tensor_walk(pps_engine* e, const pps_job_params* jp, const TensorPlan& p
   a.work = e->counters.p + CNT_TENSOR;
   a.to = to;
   a.masks = e->masks.p;
+  a.mask_cap = (uint32_t)std::min<size_t>(e->masks.n, TW_MAX_MASKS);
   debug_tensor_stall(&a.stall_at, &a.wait_limit);
   CU(launch_tensor_walk(a, e->num_sms, e->st, &e->launches));
   return PPS_OK;
@@ -935,7 +955,7 @@ static int run_job_once(pps_engine* e, const pps_job_params* jp, pps_factor* out
   if (rc) return rc;
   int variant = -1;
   TensorPlan plan;
-  const bool tensor = tensor_choice(e, jp, job_primes(e, jp), &plan);
+  const bool tensor = tensor_takes(e, jp, job_primes(e, jp), &plan);
   CU(cudaMemsetAsync(e->counters.p, 0, (tensor ? CNT_WORDS : 2u) * sizeof(uint32_t), e->st));
   if (tensor) variant = jp->sign == PPS_SIGN_TWIN ? VARIANT_TENSOR_TWIN : VARIANT_TENSOR;
   const uint64_t span = e->batch_span;
@@ -1018,18 +1038,18 @@ extern "C" int pps_run_job(pps_engine* e, const pps_job_params* jp, pps_factor* 
                            size_t* nout, pps_job_stats* st) {
   if (!e || !jp) return set_err(PPS_ERR_INVALID_PARAM, "null argument");
   if (jp->step < 1 || jp->step > 32 || jp->pmin <= (1ull << 32)) return set_err(PPS_ERR_INVALID_PARAM, "job not normalized");
+  CU(cudaSetDevice(e->device));
   if (jp->sign == PPS_SIGN_TWIN) {
     // twin jobs run on the batched walk where the tensor walk is not faster,
     // except with an input file: its rule applies on the one-job path, whose
     // twin kernels need 32-bit steps or p <= 2^(32+s)
     TensorPlan plan;
-    if (!e->input && !tensor_choice(e, jp, job_primes(e, jp), &plan)) return run_twin_job(e, jp, out, cap, nout, st);
+    if (!e->input && !tensor_takes(e, jp, job_primes(e, jp), &plan)) return run_twin_job(e, jp, out, cap, nout, st);
     bool exact = false;
     for (int v = 0; v < PPS_NUM_VARIANTS && !exact; ++v) exact = variant_ok(jp, v) != 0;
     if (!exact)
       return set_err(PPS_ERR_NOT_IMPLEMENTED, "a twin job with an input file needs 32-bit steps or p <= 2^(32+s)");
   }
-  CU(cudaSetDevice(e->device));
   size_t hit_cap = 1u << 20, fac_cap = 1u << 18;
   for (int attempt = 0; attempt < 4; ++attempt) {
     int rc = ensure_hit_buffers(e, std::max(hit_cap, e->hits.n), std::max(fac_cap, e->factors.n));
@@ -1065,7 +1085,7 @@ static int walk_device_list(pps_engine* e, const pps_job_params* jp, const uint6
                             pps_job_stats* st, bool in_range, bool* is_tensor) {
   const uint64_t*& dP = *d_list;
   TensorPlan plan;
-  const bool tensor = in_range && tensor_choice(e, jp, (double)np, &plan);
+  const bool tensor = in_range && tensor_takes(e, jp, (double)np, &plan);
   *is_tensor = tensor;
   const int variant = !tensor ? autotune(e, jp, dP, nullptr, np)
                               : jp->sign == PPS_SIGN_TWIN ? VARIANT_TENSOR_TWIN : VARIANT_TENSOR;
@@ -1077,10 +1097,12 @@ static int walk_device_list(pps_engine* e, const pps_job_params* jp, const uint6
   CU(cudaEventRecord(e->ev[2], e->st));
   cudaPointerAttributes at;
   if (tensor && cudaPointerGetAttributes(&at, dP) == cudaSuccess && at.type == cudaMemoryTypeHost) {
-    // a page-locked list: its re-check would read some primes a few times more
-    if (int rc = e->P.ensure(np)) return rc;
-    CU(cudaMemcpyAsync(e->P.p, dP, np * sizeof(uint64_t), cudaMemcpyDefault, e->st));
-    dP = e->P.p;
+    // a page-locked list: its re-check would read some primes a few times more (and
+    // does where there is no room for a copy)
+    if (e->P.ensure(np) == PPS_OK) {
+      CU(cudaMemcpyAsync(e->P.p, dP, np * sizeof(uint64_t), cudaMemcpyDefault, e->st));
+      dP = e->P.p;
+    }
   }
   const int rc = tensor ? run_tensor_walk(e, jp, plan, dP, nullptr, np, job_hits(e), true)
                         : run_walk(e, jp, variant, dP, nullptr, nullptr, np, 0, 0, (uint32_t)split);

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <map>
 #include <vector>
 
@@ -29,19 +30,19 @@ bool alloc_fault_injected();
 uint32_t debug_queue_cap();
 uint32_t debug_first_hit_cap();
 
-// Device buffer that only grows (contents are not preserved on growth).  A
-// failed growth leaves it empty (p null, n 0): whatever cached a pointer into
+// Device buffer that only grows (contents are not preserved on growth), an eighth
+// further than asked but not beyond `most`.  A failed growth leaves it empty (p null, n 0): whatever cached a pointer into
 // it must be invalidated before the call.
 template <typename T>
 struct DevBuf {
   T* p = nullptr;
   size_t n = 0;
-  int ensure(size_t want) {
+  int ensure(size_t want, size_t most = SIZE_MAX) {
     if (want <= n) return PPS_OK;
     if (p) cudaFree(p);
     p = nullptr;
     n = 0;
-    size_t grow = want + want / 8;
+    const size_t grow = std::max(want, std::min(want + want / 8, most));
     if (alloc_fault_injected())
       return set_err(PPS_ERR_INSUFFICIENT_RESOURCE, "cudaMalloc(%zu bytes): injected failure",
                      grow * sizeof(T));

@@ -780,7 +780,7 @@ cudaError_t launch_tensor_walk(TensorArgs a, int num_sms, cudaStream_t st, uint6
     ++*launches;
   }
   const uint32_t ntiles = tiles_of(a.plan);
-  uint64_t part = TW_MAX_MASKS / (a.plan.units * ntiles * 4u);  // primes of one part
+  uint64_t part = a.mask_cap / (a.plan.units * ntiles * 4u);  // primes of one part
   const uint64_t np = a.np, nparts = (np + part - 1) / part;
   part = nparts ? (np + nparts - 1) / nparts : 0;
   const uint64_t *P = a.P, *Pinv = a.Pinv;

@@ -54,6 +54,7 @@ struct TensorArgs {
   uint32_t stall_at;     // batch of each CTA before which the seeds stop (pps_debug_tensor_stall; ~0: none)
   uint4* masks;          // which rows pass: of each unit, tile and 32 rows a bit per row for columns 0-31,
                          // 32-63, 64-95 and 96-111 of the tile
+  uint32_t mask_cap;     // masks that there is room for: more primes are walked in parts
   TensorHits to;
 };
 
@@ -71,7 +72,7 @@ size_t tensor_masks(const TensorPlan& plan, uint64_t np);
 // launch's: set to each job's size, one thread's smaller job would make another's
 // launches fail.)
 cudaError_t tensor_setup();
-// The walk and the re-check of np primes, in parts of TW_MAX_MASKS masks.  *launches += the kernels launched.
+// The walk and the re-check of np primes, in parts of mask_cap masks.  *launches += the kernels launched.
 cudaError_t launch_tensor_walk(TensorArgs a, int num_sms, cudaStream_t st, uint64_t* launches);
 
 }  // namespace pps
@@ -80,6 +81,8 @@ cudaError_t launch_tensor_walk(TensorArgs a, int num_sms, cudaStream_t st, uint6
 // SM clocks per prime by the estimates.
 bool tensor_choice(const pps_engine* e, const pps_job_params* jp, double np, pps::TensorPlan* plan,
                    double* saved = nullptr);
+// Room for its masks (for a part of np primes at least), or an error.
+int ensure_masks(pps_engine* e, const pps::TensorPlan& plan, uint64_t np);
 int run_tensor_walk(pps_engine* e, const pps_job_params* jp, const pps::TensorPlan& plan, const uint64_t* dP,
                     const uint64_t* dPinv, uint64_t np, const pps::TensorHits& to, bool caller_list = false);
 // The status words in the pinned copy of the counters: an error if a wait ran
