@@ -505,6 +505,18 @@ static void fill_walk_args(const pps_job_params* jp, WalkArgs* a) {
   }
 }
 
+static int variant_ok(const pps_job_params* jp, int v);
+
+// The tensor walk's plan for a job that it can walk, in one search.
+static bool tensor_ok(const pps_job_params* jp, TensorPlan* plan) {
+  if (!tensor_plan(jp, plan)) return false;
+  if (jp->sign != PPS_SIGN_TWIN) return true;
+  // twin jobs run where a recurrence kernel could walk them too
+  for (int w = 0; w < VARIANT_TENSOR; ++w)
+    if (variant_ok(jp, w)) return true;
+  return false;
+}
+
 static int variant_ok(const pps_job_params* jp, int v) {
   const VariantTraits& t = walk_variant_traits(v);
   // the twin variants walk both sides of a twin job; every other variant one side
@@ -512,12 +524,7 @@ static int variant_ok(const pps_job_params* jp, int v) {
   if (twin != t.twin) return 0;
   if (t.tensor) {
     TensorPlan plan;
-    if (!tensor_plan(jp, &plan)) return 0;
-    if (!twin) return 1;
-    // twin jobs run where a recurrence kernel could walk them too
-    for (int w = 0; w < VARIANT_TENSOR; ++w)
-      if (variant_ok(jp, w)) return 1;
-    return 0;
+    return tensor_ok(jp, &plan);
   }
   if (t.lowbit && jp->kmax >= (1ull << 32)) return 0;  // low-bit test needs kmax < 2^32
   if (t.s32 && jp->step != 32) return 0;
@@ -739,7 +746,7 @@ bool tensor_choice(const pps_engine* e, const pps_job_params* jp, double np, Ten
   const double nsteps = (double)((jp->nmax - jp->nmin + jp->step - 1) / jp->step);
   const double old = nsteps * (twin ? 0.19 : jp->step < 32 ? 0.135 : jp->pmax <= (1ull << 47) ? 0.106 : 0.089);
   if (!forced && old < TW_LEAST_COST) return false;  // (most short jobs, without the search for a plan)
-  if (!variant_ok(jp, v) || !tensor_plan(jp, plan)) return false;
+  if (!tensor_ok(jp, plan)) return false;
   if (saved) *saved = forced ? HUGE_VAL : old - plan->cost;
   if (forced || np <= 0) return forced || plan->cost < old;
   const double primes = np / e->num_sms;  // of one SM
@@ -947,15 +954,15 @@ static int finish_job(pps_engine* e, const pps_job_params* jp, pps_factor* out, 
   return PPS_OK;
 }
 
-static int run_job_once(pps_engine* e, const pps_job_params* jp, pps_factor* out, size_t cap, size_t* nout,
-                        pps_job_stats* st, bool* overflow) {
+// plan: the tensor walk's, or null for the recurrence.
+static int run_job_once(pps_engine* e, const pps_job_params* jp, const TensorPlan* plan, pps_factor* out, size_t cap,
+                        size_t* nout, pps_job_stats* st, bool* overflow) {
   const uint32_t* dq;
   BaseTable bt;
   int rc = prepare_sieving_primes(e, jp->qmax, jp->pmax, &dq, &bt);
   if (rc) return rc;
   int variant = -1;
-  TensorPlan plan;
-  const bool tensor = tensor_takes(e, jp, job_primes(e, jp), &plan);
+  const bool tensor = plan != nullptr;
   CU(cudaMemsetAsync(e->counters.p, 0, (tensor ? CNT_WORDS : 2u) * sizeof(uint32_t), e->st));
   if (tensor) variant = jp->sign == PPS_SIGN_TWIN ? VARIANT_TENSOR_TWIN : VARIANT_TENSOR;
   const uint64_t span = e->batch_span;
@@ -982,14 +989,14 @@ static int run_job_once(pps_engine* e, const pps_job_params* jp, pps_factor* out
       variant = autotune(e, jp, e->P.p, e->Pinv.p, np);
       if (variant < 0) return variant;
     }
-    const int split = tensor ? (int)(TW_ROWS * plan.units) : choose_split(e, jp, variant, np);
+    const int split = tensor ? (int)(TW_ROWS * plan->units) : choose_split(e, jp, variant, np);
     if (split < 0) return split;
     if (st) {
       st->variant = (uint32_t)variant;
       st->split = std::max<uint32_t>(st->split, (uint32_t)split);
     }
     CU(cudaEventRecord(e->ev[2], e->st));
-    rc = tensor ? run_tensor_walk(e, jp, plan, e->P.p, e->Pinv.p, np, job_hits(e))
+    rc = tensor ? run_tensor_walk(e, jp, *plan, e->P.p, e->Pinv.p, np, job_hits(e))
                 : run_walk(e, jp, variant, e->P.p, e->Pinv.p, nullptr, np, 0, 0, (uint32_t)split);
     if (rc) return rc;
     CU(cudaEventRecord(e->ev[3], e->st));
@@ -1039,14 +1046,15 @@ extern "C" int pps_run_job(pps_engine* e, const pps_job_params* jp, pps_factor* 
   if (!e || !jp) return set_err(PPS_ERR_INVALID_PARAM, "null argument");
   if (jp->step < 1 || jp->step > 32 || jp->pmin <= (1ull << 32)) return set_err(PPS_ERR_INVALID_PARAM, "job not normalized");
   CU(cudaSetDevice(e->device));
-  if (jp->sign == PPS_SIGN_TWIN) {
+  TensorPlan plan;
+  const bool tensor = tensor_takes(e, jp, job_primes(e, jp), &plan);
+  if (jp->sign == PPS_SIGN_TWIN && !tensor) {
     // twin jobs run on the batched walk where the tensor walk is not faster,
     // except with an input file: its rule applies on the one-job path, whose
     // twin kernels need 32-bit steps or p <= 2^(32+s)
-    TensorPlan plan;
-    if (!e->input && !tensor_takes(e, jp, job_primes(e, jp), &plan)) return run_twin_job(e, jp, out, cap, nout, st);
+    if (!e->input) return run_twin_job(e, jp, out, cap, nout, st);
     bool exact = false;
-    for (int v = 0; v < PPS_NUM_VARIANTS && !exact; ++v) exact = variant_ok(jp, v) != 0;
+    for (int v = 0; v < VARIANT_TENSOR && !exact; ++v) exact = variant_ok(jp, v) != 0;
     if (!exact)
       return set_err(PPS_ERR_NOT_IMPLEMENTED, "a twin job with an input file needs 32-bit steps or p <= 2^(32+s)");
   }
@@ -1058,7 +1066,7 @@ extern "C" int pps_run_job(pps_engine* e, const pps_job_params* jp, pps_factor* 
     if (st) memset(st, 0, sizeof *st);
     bool overflow = false;
     cudaEventRecord(e->ev[6], e->st);
-    rc = run_job_once(e, jp, out, cap, nout, st, &overflow);
+    rc = run_job_once(e, jp, tensor ? &plan : nullptr, out, cap, nout, st, &overflow);
     if (rc) return rc;
     if (!overflow) {
       cudaEventRecord(e->ev[7], e->st);
