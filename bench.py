@@ -18,10 +18,11 @@ e2e    = the same metric through the drop-in C-ABI call with HOST buffers:
          the host link by the recurrence, inside the timed region) and
          returning the factor list to the host (D2H inside the timed region) --
          what the reference's check_ns / get_factors_found boundary carries.
-roofline: the tensor walk is bound by the issue of instructions; its work is the
-         warp instructions per prime of its committed profile, the peak four a
-         clock and SM at the clock sampled in this run; beside it the rate of its
-         matrix products.  The recurrence is bound by the 32-bit integer
+roofline: the tensor walk's work is its matrix products, the peak the measured
+         tensor rate.  What bounds it is the issue of instructions: beside that,
+         how busy the issue slots are (the kernel's own instructions per prime, of
+         its committed profile, over four a clock and SM at the clock sampled in
+         this run), which says nothing of a floor.  The recurrence is bound by the 32-bit integer
          multiply pipe; its algorithmic work is 3 multiplies per walk step (one
          32 n-values advance of one prime); the peak is the multiply-pipe
          throughput measured in this run by pps_measure_imad_peak on the same
@@ -163,6 +164,22 @@ def _from_profile(kernel: str, key: str = "dram_bytes_per_prime") -> float | Non
         if line.startswith(key + ":"):
             return float(line.split(":")[1])
     return None
+
+
+def _tensor_roofline(kernel: str, rate: float, sm_mhz: float, sms: int, tflops: float | None) -> dict:
+    """The tensor walk at `rate` primes/s: its matrix products against the measured
+    tensor rate, and the share of the issue slots that its own instructions take
+    (polls of its waits among them, so no measure of how near it is to a floor)."""
+    flop = _from_profile(kernel, "mma_flop_per_prime") or 0.0
+    instr = _from_profile(kernel, "warp_instructions_per_prime") or 0.0
+    done, slots = flop * rate / 1e12, 4.0 * sm_mhz * 1e6 * sms
+    return {"bound": "tensor", "achieved": done, "peak": tflops, "unit": "TFLOP/s",
+            "frac": done / tflops if tflops else None,
+            "peak_source": "MEASURED_PEAKS.json bf16_tflops (of measured)",
+            "work_per_unit": f"{flop:.0f} flop of fp16 matrix products per prime",
+            "issue_slots": {"busy": instr * rate / slots if slots else None,
+                            "warp_instructions_per_prime": instr,
+                            "peak_source": "4 a clock and SM at the median SM clock of this run"}}
 
 
 def _measured_peaks() -> dict:
@@ -880,30 +897,22 @@ def run_gpu(args) -> None:
     kernel = ppsgpu.walk_kernel_name(variant)
     traffic = _from_profile(kernel)
     peaks = _measured_peaks()
-    tensor = None
     if kernel == "k_tensor_walk":
-        instr, flop = _from_profile(kernel, "warp_instructions_per_prime"), _from_profile(kernel, "mma_flop_per_prime")
+        sms = torch.cuda.get_device_properties(local).multi_processor_count
         mhz = clk.summary()["sm_mhz"] or peaks.get("sm_max_mhz") or 0.0
-        bound, unit, per = "issue", "G warp instructions/s", f"{instr} warp instructions per prime (ncu)"
-        achieved, peak = (instr or 0.0) * primes / (walk_ms * 1e-3), 4.0 * mhz * 1e6 * torch.cuda.get_device_properties(local).multi_processor_count
-        source = "4 a clock and SM at the median SM clock of this run"
-        rate, tf = (flop or 0.0) * primes / (walk_ms * 1e-3) / 1e12, peaks.get("bf16_tflops")
-        tensor = {"bound": "tensor", "achieved": rate, "peak": tf, "unit": "TFLOP/s", "frac": rate / tf if tf else None,
-                  "peak_source": "MEASURED_PEAKS.json bf16_tflops (of measured)",
-                  "work_per_unit": f"{flop} flop of fp16 matrix products per prime"}
+        roof = _tensor_roofline(kernel, primes / (walk_ms * 1e-3), mhz, sms, peaks.get("bf16_tflops"))
     else:
-        bound, unit, per = "imad", "Gmul/s", "3 multiplies per walk step (one prime advanced by 32 n)"
         achieved, peak = 3.0 * steps_done / (walk_ms * 1e-3), eng.imad_peak()
-        source = "measured in this run (pps_measure_imad_peak)"
+        roof = {"bound": "imad", "achieved": achieved / 1e9, "peak": peak / 1e9, "unit": "Gmul/s",
+                "frac": achieved / peak, "peak_source": "measured in this run (pps_measure_imad_peak)",
+                "work_per_unit": "3 multiplies per walk step (one prime advanced by 32 n)"}
     hbm = peaks.get("hbm_gbs")
     sieve_gbs = 16.0 * primes / (sieve_ms * 1e-3) / 1e9 if sieve_ms > 0 else None
     walks = len(stats)  # one walk per job (the tensor walk in several launches)
-    roofline = {"bound": bound, "achieved": achieved / 1e9, "peak": peak / 1e9,
-                "unit": unit, "frac": achieved / peak if peak else None,
+    roofline = {**roof,
                 "traffic": (traffic * primes / walks) if traffic else None,
                 "traffic_unit": "bytes per walk of a slice (ncu DRAM bytes per prime x its primes)",
                 "kernel": f"{kernel} (variant {variant}: {ppsgpu.walk_variant_name(variant)})",
-                "peak_source": source, "work_per_unit": per, "tensor": tensor,
                 "sieve": {"bound": "hbm", "achieved": sieve_gbs, "peak": hbm, "unit": "GB/s",
                           "frac": (sieve_gbs / hbm) if (sieve_gbs and hbm) else None,
                           "peak_source": "MEASURED_PEAKS.json hbm_gbs (of measured)",

@@ -33,3 +33,16 @@ def test_reference_legs_absent_without_a_build(tmp_path):
     assert b.reference_gpu_sample(None, binary=tmp_path / "missing_dropin") is None
     b.REF_BIN = tmp_path / "missing_cpu"
     assert b.reference_sample(1.0) is None
+
+
+def test_tensor_roofline_is_work_over_a_measured_peak(monkeypatch):
+    """The fraction is the matrix products' (fixed by the method) and does not move
+    with the kernel's own instruction count, which only says how busy it is."""
+    b = _bench()
+    rows = []
+    for instr in (4000.0, 2000.0):
+        monkeypatch.setattr(b, "_from_profile", lambda _, key, i=instr: {"mma_flop_per_prime": 3.0e6}.get(key, i))
+        rows.append(b._tensor_roofline("k_tensor_walk", 2.0e8, 2000.0, 100, 1500.0))
+    assert rows[0]["bound"] == "tensor" and abs(rows[0]["frac"] - 0.4) < 1e-12
+    assert rows[0]["frac"] == rows[1]["frac"]
+    assert abs(rows[0]["issue_slots"]["busy"] - 1.0) < 1e-12 and abs(rows[1]["issue_slots"]["busy"] - 0.5) < 1e-12
