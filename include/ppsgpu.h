@@ -193,7 +193,8 @@ int pps_run_job(pps_engine *e, const pps_job_params *jp, pps_factor *out,
 /* Walk a caller-supplied list of primes held in HOST memory.  A page-locked
    (pinned) buffer, e.g. from cudaHostAlloc, is read in place by the recurrence
    over the host link; the tensor walk, and any other buffer, has it copied to
-   the device inside the call.  A
+   the device inside the call (the tensor walk reads it in place too where there
+   is no room for the copy).  A
    list that starts in page-locked memory must lie in one page-locked
    allocation or registration (cudaHostRegister) for its whole length.  Same
    output rule and order as pps_run_job. */
@@ -279,7 +280,10 @@ int pps_engine_set_input(pps_engine *e, const pps_input *in);
    chunks of primes from a device work counter; each wave's launch sequence is
    a captured CUDA graph; the work per chunk (walk steps per lane: a job's
    chunk holds work*32/nsteps primes) and the unroll are tuned on the first
-   wave and reported in `chunk` and `unroll`.  Factors come back grouped by
+   wave that the walk kernel has work in.  `chunk` and `unroll` report those of
+   the last wave: a wave with too little work for the GPU takes smaller chunks
+   than the tuned ones, and where the tensor walk took every job they stand at
+   1024 and 8.  Factors come back grouped by
    job (job_offsets[j]..job_offsets[j+1]), each group sorted by (p, k, n),
    exactly as pps_run_job would return them. */
 typedef struct {

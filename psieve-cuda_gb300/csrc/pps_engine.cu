@@ -722,21 +722,22 @@ static int autotune(pps_engine* e, const pps_job_params* jp, const uint64_t* dP,
 
 // Whether the job runs on the tensor walk, and how: where its cost is estimated
 // to be below the recurrence's, both in SM clocks per prime.  tensor_plan's
-// estimate holds within 9%.  The recurrence's is its steps times what one took
-// with 1.5 to 2.4 million primes: 32-bit steps 0.106-0.110 (p up to 2^50;
-// 0.089 at 2^62), shorter ones 0.135, a twin step 0.19-0.24 (on the batched
-// form).  On either side of the line: p = 4.2e13, N = 200,000: 692 clocks
-// against the tensor walk's 714, N = 250,000: 861 against 740; p = 2^62, N =
-// 250,000: 711 against 761, N = 300,000: 852 against 784; p = 10^12, N =
-// 131,071: 669 against 713, N = 150,000: 764 against 724.
+// estimate is up to 12% high.  The recurrence's is its steps times what one took
+// with 2 million primes: 32-bit steps 0.106-0.110 (p up to 2^50; 0.087 at 2^62,
+// whose figure every p above 2^47 gets), shorter ones 0.135, a twin step
+// 0.19-0.24 (on the batched form).  On either side of the line: p = 4.2e13, N =
+// 200,000: 691 clocks and the tensor walk's 689, N = 250,000: 856 and 708; p =
+// 2^62, N = 250,000: 686 and 730, N = 300,000: 823 and 747; p = 10^12, N =
+// 131,071: 671 and 686, N = 150,000: 767 and 697.
 // With few primes (np > 0) the calls' times decide: the tensor walk's launches,
-// first seeds and tail are about 55,000 clocks (27 us), its share of the call's
-// host time 5 us more; the recurrence takes a fifth longer on less than a third
-// of its resident threads, and cannot be faster than one thread's eighth of the
-// n range, 58 clocks a step (38 for the shorter steps).  Over 252 calls of 300
-// to 400,000 primes and 100,000 to 700,000 n this takes the slower walk nowhere
-// by more than the calls' own spread; by the estimates above alone 3,000 primes
-// at 10^12, 150,000 n took 27 us instead of 22.
+// first seeds and tail are about 55,000 clocks (27 us), 11,000 more were its
+// share of the call's host time (it is less now); the recurrence takes a fifth
+// longer on less than a third of its resident threads, and cannot be faster than
+// one thread's eighth of the n range, 58 clocks a step (38 for the shorter steps).
+// The rule errs towards the recurrence: of 252 calls of 300 to 400,000 primes and
+// 100,000 to 700,000 n it gives 109 to the tensor walk, each at least 10% faster
+// so, and of the 143 others 56 would be 3% to 57% faster on it.  By the estimates
+// above alone 3,000 primes at 10^12, 150,000 n took 27 us instead of 22.
 bool tensor_choice(const pps_engine* e, const pps_job_params* jp, double np, TensorPlan* plan, double* saved) {
   const bool twin = jp->sign == PPS_SIGN_TWIN;
   const int v = twin ? VARIANT_TENSOR_TWIN : VARIANT_TENSOR;

@@ -49,13 +49,13 @@
 //                   pass in each 32 columns: a mask to global memory
 // and a second kernel, one thread to a passing row.
 //
-// Measured, 8.56 million primes at 4.2e13, a million n: 38.7 ms, of which the
+// Measured, 8.56 million primes at 4.2e13, a million n: 38.4 ms, of which the
 // second kernel 10%, against 91.0 ms of the recurrence; 6.24 million at 2^62,
-// 900,000 n: 22.3 against 47.9 ms.  What bounds the first kernel is the issue
-// of instructions (3,460 a prime, 71% of the slots, the integer pipe 73% busy),
-// no longer multiplies: about 90 a warp and test tile, of them 32 the minima,
-// 45 a B row warp, 190 an A warp.  Its chains come close behind: the build warps
-// spend 60% of a prime's 1,300 clocks on their rows (a third group took the
+// 900,000 n: 22.1 against 47.9 ms.  What bounds the first kernel is the issue
+// of instructions (3,390 a prime, 72% of the slots, the integer pipe 73% busy),
+// no longer multiplies: 79 a warp and test tile beside its waits, of them 32 the
+// minima, 48 to 32 B rows, 138 to 32 A rows.  Its chains come close behind: the
+// build warps spend 60% of a prime's 1,270 clocks on their rows (a third group took the
 // cases above from 41.7 and 26.7 ms), a test warp 70% on its tile.  The MMAs
 // fill 224 clocks.  A tile in one load, which frees it sooner but holds 24
 // registers more, made no difference.
@@ -711,8 +711,9 @@ size_t tensor_smem(uint32_t nb, uint32_t pitch) {
 
 // For each number of units the columns and the stride that cover the n range,
 // by an estimate of the SM clocks per prime: set-up and A rows per unit, B rows
-// and tests per column and tile, and the re-check of what passes.  Fitted to 48
-// sizes from 30,000 to 2 million n at p = 10^12 to 2^62, within 9% of each.
+// and tests per column and tile, and the re-check of what passes.  For 48 sizes
+// from 30,000 to 2 million n at p = 10^12 to 2^62 it lies between 2% below and 12%
+// above the time that they took.
 bool tensor_plan(const pps_job_params* jp, TensorPlan* out) {
   if (jp->nmax <= jp->nmin || jp->nmin < 128u || jp->pmin <= (1ull << 32) || jp->pmax > (1ull << 62)) return false;
   if (jp->pmax <= jp->pmin || jp->kmax < jp->kmin) return false;
